@@ -172,10 +172,7 @@ typedef struct tfg_engine_desc {
  *   volume 0).  The first step after a load, a boundary change or a change of a batch's
  *   membership rebuilds.  The displacement is measured as the
  *   reference's OpenMP branch measures it; its default branch discards it (the sum goes to
- *   a shadowing int), so the reference itself never rebuilds after the first step.  On the
- *   device, the rebuild step also records each home cell's interacting-pair candidates
- *   within the skin radius, and the other steps evaluate those lists instead of testing
- *   every candidate pair. */
+ *   a shadowing int), so the reference itself never rebuilds after the first step. */
 #define TFG_ENGINE_DPD_REFERENCE_RANDOM (1u << 0)
 #define TFG_ENGINE_NO_DENSITY           (1u << 1)
 #define TFG_ENGINE_VERLET               (1u << 2)
@@ -293,20 +290,17 @@ TFG_API int tfg_query(tfg_engine *eng, int *idle);
  * split or stream one step runs eagerly, and the following steps replay a captured
  * single-step graph (one per particle-buffer parity), phase events included. */
 TFG_API int tfg_set_graphs(tfg_engine *eng, int enable);
-/* Pair lists for simulations in Verlet mode (default on): the tiled pass records each home
- * cell's pairs within the list radius at a rebuild and evaluates those lists until the
- * next one; off, every step tests all candidate pairs of the cell stencil.  The pair set
- * is the same either way. */
+/* Accepted for callers that switch pair lists of simulations in Verlet mode on or off; has no
+ * effect: every step tests the candidate pairs of the cell stencil, which is faster than
+ * walking recorded lists.  The pair set is the same either way. */
 TFG_API int tfg_set_pair_lists(tfg_engine *eng, int enable);
 /* Autotune the nonbonded pass's form by timing each choice on the current state; the
  * state is left unchanged.  The choices are the tiled kernel's work split (warps per home
- * cell: 1, 2, 7 or 14) and, for engines whose potentials are all tabulated (no DPD, no
- * fluxes, no Verlet pair lists), TFG_PAIR_HOME_OUTER: the kernel that takes home particles
- * one at a time against targets held in registers.  tfg_step and tfg_force_only run it on
- * their first call, and time the work splits again whenever the particle count has grown
- * or shrunk more than 4x since (a batch that fills up or drains); tfg_set_split fixes the
- * choice instead (TFG_PAIR_HOME_OUTER falls back
- * to split 1 while the engine is not eligible).  The reference selects CUDA
+ * cell: 1, 2, 7 or 14), its warps per CTA and its smallest grab of work items.  tfg_step and
+ * tfg_force_only run it on their first call, and time the work splits again whenever the
+ * particle count has grown or shrunk more than 4x since (a batch that fills up or drains);
+ * tfg_set_split fixes the choice instead (TFG_PAIR_HOME_OUTER, once a kernel of its own, is
+ * accepted and runs as split 1).  The reference selects CUDA
  * blocks/threads by hand (cuda::EngineConfig::setBlocks / setThreads,
  * source/cuda/tfEngineConfig.cpp:98-124). */
 #define TFG_PAIR_HOME_OUTER 32
@@ -322,9 +316,7 @@ TFG_API int tfg_set_tuning(tfg_engine *eng, int split, int warps_per_cta, int gr
 /* Pair-set signature of the current binned state, per particle id: the number of
  * partners with r2 <= cutoff^2 and the wrap-around sum of a 32-bit mix of their ids.
  * It runs the pair pass's own stencil walk and pair decision (no forces).  Call it after
- * tfg_force_only to describe the pair set that pass used.  A simulation in Verlet mode
- * that did not rebuild at its last step is walked through its pair lists, as its next
- * force pass would be.  Verification hook; the reference has no counterpart. */
+ * tfg_force_only to describe the pair set that pass used.  Verification hook; the reference has no counterpart. */
 TFG_API int tfg_pair_signature(tfg_engine *eng, int32_t *count, uint32_t *hash);
 /* The interacting pairs themselves, from the same kernels and pair decision as
  * tfg_pair_signature: up to cap pairs (lower id, higher id), 2*cap ints, in no particular

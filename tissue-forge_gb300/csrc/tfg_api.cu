@@ -43,14 +43,14 @@ int make_engine(int device, int max_type, int nspec, tfg_engine **out) {
     for (auto &p : eng->h_bpots) std::memset(&p, 0, sizeof(p));
     eng->h_btables.assign(kMaxBondSlots, std::vector<float>());
     int rc;
-    if ((rc = dalloc(eng, &eng->err, 2)) || (rc = dalloc(eng, &eng->overflow_count, 2)) ||
+    if ((rc = dalloc(eng, &eng->err, 2)) || (rc = dalloc(eng, &eng->counters, 4)) ||
         (rc = dalloc(eng, &eng->bpots, kMaxBondSlots)) || (rc = dalloc(eng, &eng->stamps, 5))) {
         destroy(eng);
         return rc;
     }
     eng->err_slots = 1;
     cudaMemset(eng->err, 0, 2 * sizeof(uint32_t));
-    cudaMemset(eng->overflow_count, 0, 2 * sizeof(int));
+    cudaMemset(eng->counters, 0, 4 * sizeof(unsigned));
     cudaMemset(eng->stamps, 0, sizeof(unsigned long long) * 5);
     if (cudaDeviceSynchronize() != cudaSuccess) {
         destroy(eng);
@@ -416,9 +416,7 @@ TFG_API int tfg_force_only(tfg_engine *eng, int with_bonded) {
     int rc = commit(eng);
     if (rc) return rc;
     if ((rc = tune_if_needed(eng))) return rc;
-    cudaStream_t s = eng->stream;
     advance_clocks(eng);
-    launch_tick((int)eng->order.size(), eng->sims_dev, eng->red, s);
     rc = bin(eng, 1);
     if (rc) return rc;
     return force_pass(eng, with_bonded != 0, false);
@@ -452,8 +450,7 @@ static int signature_pass(tfg_engine *eng, int32_t *count, uint32_t *hash, int64
     }
     cudaMemsetAsync(dbuf, 0, sizeof(int32_t) * (words + 1), eng->stream);
     if (use_tile(eng))
-        launch_pair_tile(a, tile_plan(eng, eng->split), eng->overflow_list, eng->overflow_count, eng->sms, true,
-                         tune_of(eng), eng->stream);
+        launch_pair_tile(a, eng->sms, true, tune_of(eng), eng->stream);
     else
         launch_pair_signature(a, eng->stream);
     if (count) cudaMemcpyAsync(count, a.sig_count, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, eng->stream);
@@ -531,7 +528,7 @@ TFG_API int tfg_batch_get_reductions(tfg_engine *eng, int sim, tfg_reductions *o
 }
 TFG_API int tfg_set_pair_lists(tfg_engine *eng, int enable) {
     if (!eng) return TFG_E_INVAL;
-    eng->lists_wanted = enable != 0;   // applied at the next step; lists fill at the next rebuild
+    (void)enable;   // Verlet mode tests its candidate pairs every step, with the same pair set
     return TFG_OK;
 }
 TFG_API int tfg_get_verlet(tfg_engine *eng, int64_t *rebuilds, float *maxdx) {

@@ -48,6 +48,16 @@ struct __align__(16) PotDev {
 static_assert(sizeof(PotDev) == 64, "PotDev layout");
 enum : uint32_t { POT_NONE = 0, POT_TABLE = 1, POT_DPD = 2 };
 
+// The same potential as the tiled pair pass reads it, in two 128-bit loads per pair.
+struct __align__(16) PotPair {
+    float p0, p1, p2, b;   // table: alpha0..2; DPD: alpha, gamma, sigma
+    float a, c;            // c: r0_plusone (table), 1/b (DPD)
+    uint32_t nk;           // table intervals n | POTC_* bits
+    int32_t offset;        // as PotDev
+};
+static_assert(sizeof(PotPair) == 32 && TFG_POTENTIAL_IVALSMAX < 65536, "PotPair layout");
+enum : uint32_t { POTC_TABLE = 1u << 16, POTC_DPD = 1u << 17, POTC_SHIFTED = 1u << 18, POTC_SCALED = 1u << 19 };
+
 struct FluxDev {
     int32_t kind, type_a, type_b, index_a, index_b;
     float coef, half_decay, target, cutoff;
@@ -70,6 +80,11 @@ struct SimParams {
     int32_t cell_off, id_off, angle_off;
     int32_t pot_base, type_base, red_base, spec_base;
     float cutoff, cutoff2;
+    // Bound of the tiled pair pass's distance filter x_i - (x_k + shift) above cutoff2.  Each
+    // component of it and of the reference's (x_i - shift) - x_k is rounded at a magnitude of
+    // at most twice the cell edge h, so the squares at the cutoff differ by less than
+    // 1.3e-6 h/cutoff + 5e-7 relative; the bound keeps four times that.
+    float cut_hi;
     float dt, dt_flux;
     float maxx[3], maxx2[3], maxv[3], maxv2[3], h2[3];
     float inv_cutoff;        // 1/cutoff in FP32
@@ -99,8 +114,7 @@ struct SimParams {
     // device fields are written by k_tick and k_advance; the host writes 2 to
     // verlet_rebuild to force a rebuild at the next step.
     float skin;              // min(h) - cutoff
-    float rlist2;            // (cutoff + skin)^2 with a relative margin: pair-list radius
-    int32_t verlet_rebuild;  // device: this step re-bins and rebuilds the pair lists
+    int32_t verlet_rebuild;  // device: this step re-bins
     uint32_t verlet_maxdx2;  // device: max |x - oldx|^2 after the last advance (float bits)
     float verlet_maxdx;      // device: largest displacement at the last check (0 on a rebuild)
     int64_t verlet_rebuilds; // device: rebuilds so far
@@ -161,7 +175,7 @@ __device__ __forceinline__ float gauss_pair(uint64_t seed, int64_t step, int ida
     int lo = min(ida, idb), hi = max(ida, idb);
     U4 r = philox({(uint32_t)step, (uint32_t)lo, (uint32_t)hi, STREAM_DPD}, (uint32_t)seed, (uint32_t)(seed >> 32));
     float u1 = u01(r.x), u2 = u01(r.y);
-    return sqrtf(-2.0f * logf(u1)) * cosf(6.283185307179586f * u2);
+    return sqrtf(-2.0f * logf(u1)) * cospif(2.0f * u2);
 }
 
 // Normal deviate of the DPD wall random term, keyed on (step, particle, wall).

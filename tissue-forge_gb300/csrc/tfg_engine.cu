@@ -2,7 +2,7 @@
 // reductions.  One step over the arena (engine_step, tfEngine.cpp:1378-1429):
 //   tick     every simulation's time += 1 (on the device)
 //   bin      space_shuffle_local re-check + counting sort into cell order
-//   pair     fused nonbonded pass (tfg_pair_tile.cu, or tfg_pair.cu for several species)
+//   pair     fused nonbonded pass (tfg_pair_tile.cu, or tfg_pair.cu in deterministic mode)
 //   bonded   bond_eval / angle_eval
 //   advance  forward Euler + Fluxes_integrate + FP64 per-simulation totals
 #include <algorithm>
@@ -41,6 +41,9 @@ int alloc_particles(tfg_engine *eng, ParticleArrays &A, int cap) {
         (rc = dalloc(eng, &A.fext, cap)) || (rc = dalloc(eng, &A.pforce, cap)) || (rc = dalloc(eng, &A.cell, cap)) ||
         (rc = dalloc(eng, &A.sval, (size_t)cap * ns)) || (rc = dalloc(eng, &A.sq, (size_t)cap * ns)))
         return rc;
+    // both copies start at zero: they are not moved while no simulation has such a force
+    CK(cudaMemsetAsync(A.fext, 0, sizeof(float4) * cap, eng->stream));
+    CK(cudaMemsetAsync(A.pforce, 0, sizeof(float4) * cap, eng->stream));
     return TFG_OK;
 }
 
@@ -212,8 +215,7 @@ int relayout(tfg_engine *eng) {
         eng->cur = 0;
         int r2;
         if ((r2 = dalloc(eng, &eng->force, new_cap)) || (r2 = dalloc(eng, &eng->lidx, new_cap)) ||
-            (r2 = dalloc(eng, &eng->tmp_id, new_cap)) || (r2 = dalloc(eng, &eng->tmp_src, new_cap)) ||
-            (r2 = dalloc(eng, &eng->dest, new_cap)) || (r2 = dalloc(eng, &eng->slot_of_id, new_cap)))
+            (r2 = dalloc(eng, &eng->bin_tmp, new_cap)) || (r2 = dalloc(eng, &eng->slot_of_id, new_cap)))
             return r2;
         eng->cap = new_cap;
     } else {
@@ -251,11 +253,13 @@ int relayout(tfg_engine *eng) {
     if (C + 1 > eng->cells_cap) {
         const int cc = C + 1;
         if ((rc = dalloc(eng, &eng->count, cc)) || (rc = dalloc(eng, &eng->start, cc + 1)) ||
-            (rc = dalloc(eng, &eng->scan_sums, (cc + 1023) / 1024 + 1)) || (rc = dalloc(eng, &eng->cell_sim, cc)) ||
-            (rc = dalloc(eng, &eng->overflow_list, cc)))
+            (rc = dalloc(eng, &eng->scan_part, cc)) || (rc = dalloc(eng, &eng->scan_pre, scan_blocks(cc) + 1)) ||
+            (rc = dalloc(eng, &eng->cell_sim, cc)))
             return rc;
+        CK(cudaMemsetAsync(eng->count, 0, sizeof(int32_t) * cc, s));
         eng->cells_cap = cc;
     }
+    if ((rc = ensure(eng, &eng->items, eng->items_cap, (size_t)C + N / 32 + 1))) return rc;
     CK(cudaMemcpyAsync(eng->cell_sim, cell_sim.data(), sizeof(int32_t) * std::max(C, 1), cudaMemcpyHostToDevice, s));
     if ((int)order.size() > eng->err_slots) {
         const int slots = std::max((int)order.size(), 2 * eng->err_slots);
@@ -321,6 +325,25 @@ int relayout(tfg_engine *eng) {
     return TFG_OK;
 }
 
+// A potential in the tiled pair pass's compact form.
+PotPair to_pair(const PotDev &p) {
+    PotPair c;
+    std::memset(&c, 0, sizeof(c));
+    if (p.kind == POT_NONE) return c;
+    const bool table = p.kind == POT_TABLE;
+    c.p0 = table ? p.alpha0 : p.dpd_alpha;
+    c.p1 = table ? p.alpha1 : p.dpd_gamma;
+    c.p2 = table ? p.alpha2 : p.dpd_sigma;
+    c.b = p.b;
+    c.a = p.a;
+    c.c = table ? p.r0_plusone : 1.0f / p.b;
+    c.nk = table ? (uint32_t)p.n | POTC_TABLE : (uint32_t)POTC_DPD;
+    if (p.flags & TFG_POTENTIAL_SHIFTED) c.nk |= POTC_SHIFTED;
+    if (table && (p.flags & TFG_POTENTIAL_SCALED)) c.nk |= POTC_SCALED;
+    c.offset = p.offset;
+    return c;
+}
+
 // Upload the interaction tables of every live simulation (potentials with their table
 // blob, fluxes, per-type arrays, species flags) and the bonded potentials.
 int upload_tables(tfg_engine *eng) {
@@ -371,6 +394,7 @@ int upload_tables(tfg_engine *eng) {
         }
         for (int t = 0; t < T; t++) {
             rf[q * T + t] = S.rforce[t];
+            eng->has_rand |= rf[q * T + t].w != 0.f;
             mass[q * T + t] = S.mass[t];
             dyn[q * T + t] = S.dyn[t];
         }
@@ -396,6 +420,10 @@ int upload_tables(tfg_engine *eng) {
         (rc = ensure(eng, &eng->species_flags, eng->spec_cap, spf.size())) ||
         (rc = ensure(eng, &eng->wpots, eng->wpots_cap, wp.size())))
         return rc;
+    std::vector<PotPair> pc(pots.size());
+    for (size_t k = 0; k < pots.size(); k++) pc[k] = to_pair(pots[k]);
+    if ((rc = ensure(eng, &eng->potc, eng->potc_cap, pc.size()))) return rc;
+    CK(cudaMemcpyAsync(eng->potc, pc.data(), sizeof(PotPair) * pc.size(), cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(eng->wpots, wp.data(), sizeof(PotDev) * wp.size(), cudaMemcpyHostToDevice, s));
     if (rf.size() > eng->types_cap) {
         if ((rc = dalloc(eng, &eng->rforce, rf.size())) || (rc = dalloc(eng, &eng->type_mass, rf.size())) ||
@@ -612,6 +640,7 @@ int add_sim(tfg_engine *eng, const tfg_engine_desc *d, int *out) {
     P.ncells = P.cdim[0] * P.cdim[1] * P.cdim[2];
     P.cutoff = d->cutoff;
     P.cutoff2 = d->cutoff * d->cutoff;
+    P.cut_hi = P.cutoff2 * (1.f + 2e-6f + 5e-6f * (std::max(P.h[0], std::max(P.h[1], P.h[2])) / P.cutoff));
     P.dt = d->dt;
     const float frac = d->particle_max_dist_fraction > 0 ? d->particle_max_dist_fraction : 0.05f;
     for (int k = 0; k < 3; k++) {
@@ -632,9 +661,6 @@ int add_sim(tfg_engine *eng, const tfg_engine_desc *d, int *out) {
     P.seed = d->seed;
     // engine_verlet_update (tfEngine.cpp:231): skin = min(h) - cutoff, in FP32
     P.skin = std::fmin(P.h[0], std::fmin(P.h[1], P.h[2])) - P.cutoff;
-    // a pair within the cutoff after both partners moved at most skin/2 was within
-    // cutoff + skin at the rebuild; the margin covers the FP32 rounding of r2
-    P.rlist2 = (P.cutoff + P.skin) * (P.cutoff + P.skin) * 1.0001f;
     P.verlet_rebuild = 2;
     P.stop_at = -1;
     S.maxc = std::max(P.cdim[0], std::max(P.cdim[1], P.cdim[2]));
@@ -694,6 +720,10 @@ int load_sim(tfg_engine *eng, int sim, int n, const float *xg, const int32_t *ce
     cp(S.imass, imass, n);
     cp(S.species, species, (size_t)n * ns);
     cp(S.force_i, force_i, (size_t)3 * n);
+    if (force_i && !eng->has_ext) {
+        eng->has_ext = true;
+        eng->gen++;
+    }
     S.type.assign(n, 0);
     if (type) std::memcpy(S.type.data(), type, sizeof(int32_t) * n);
     if (flags) S.flags.assign(flags, flags + n);
@@ -723,11 +753,17 @@ int bin(tfg_engine *eng, int shuffle) {
     b.count = eng->count;
     b.start = eng->start;
     b.lidx = eng->lidx;
-    b.tmp_id = eng->tmp_id;
-    b.tmp_src = eng->tmp_src;
-    b.dest = eng->dest;
-    b.scan_sums = eng->scan_sums;
-    b.slot_of_id = eng->slot_of_id;
+    b.slot_of_id = eng->nb + eng->na > 0 ? eng->slot_of_id : nullptr;
+    b.tmp = eng->bin_tmp;
+    b.part = eng->scan_part;
+    b.pre = eng->scan_pre;
+    b.ticket = eng->counters;
+    b.items = eng->items;
+    b.nitems = reinterpret_cast<int *>(eng->counters + 1);
+    b.nsims = (int)eng->order.size();
+    b.red = eng->red;
+    b.has_ext = eng->has_ext;
+    b.has_rand = eng->has_rand;
     b.rforce = eng->rforce;
     b.force = eng->force;
     b.oldx = eng->oldx;
@@ -748,97 +784,6 @@ int commit(tfg_engine *eng) {
         CK(cudaStreamSynchronize(eng->stream));
         if ((rc = check_launch(eng))) return rc;
     }
-    return prepare_lists(eng, relaid);
-}
-
-namespace {
-
-// Entries per home cell for the Verlet pair lists: twice the mean half-shell pair count
-// within the list radius of the densest simulation, plus room for the chunk markers.
-int estimate_list_k(const tfg_engine *eng) {
-    double best = 0.0;
-    for (int k : eng->order) {
-        const SimHost &S = eng->sims[k];
-        if (!(S.P.flags & TFG_ENGINE_VERLET) || S.n == 0) continue;
-        const double vol = (double)S.P.dim[0] * S.P.dim[1] * S.P.dim[2];
-        const double rl = (double)S.P.cutoff + S.P.skin;
-        const double per_cell = (double)S.n / S.P.ncells;
-        best = std::max(best, per_cell * (S.n / vol) * (2.0 / 3.0) * 3.14159265358979 * rl * rl * rl);
-    }
-    const int k = (int)std::ceil(2.0 * best) + 4 * 128;   // chunks start 128-entry groups
-    return (k + 127) & ~127;
-}
-
-// Pair lists take at most this many bytes; cells whose list does not fit under it keep
-// testing candidate pairs.
-constexpr size_t kMaxListBytes = size_t(16) << 30;
-
-int capped_list_k(const tfg_engine *eng, int k) {
-    const size_t cells = (size_t)std::max(eng->ncells, 1);
-    const size_t most = kMaxListBytes / sizeof(uint32_t) / cells;
-    return (int)std::min<size_t>((size_t)k, std::max<size_t>(most & ~size_t(127), 128));
-}
-
-int alloc_lists(tfg_engine *eng) {
-    const size_t cells = (size_t)std::max(eng->ncells, 1);
-    int rc;
-    if ((rc = ensure(eng, &eng->vlen, eng->vlen_cap, cells)) ||
-        (rc = ensure(eng, &eng->vlist, eng->vlist_cap, cells * (size_t)eng->list_k)))
-        return rc;
-    CK(cudaMemsetAsync(eng->vlen, 0xff, sizeof(int32_t) * cells, eng->stream));   // -1: no list
-    return TFG_OK;
-}
-
-}  // namespace
-
-int prepare_lists(tfg_engine *eng, bool relaid) {
-    bool any = false;
-    for (int k : eng->order) any |= (eng->sims[k].P.flags & TFG_ENGINE_VERLET) != 0;
-    const bool use = any && eng->lists_wanted && use_tile(eng) && !eng->has_dpd && !(eng->has_flux && eng->nspec > 0);
-    if (!use) {
-        if (eng->lists_on) eng->gen++;
-        eng->lists_on = false;
-        return TFG_OK;
-    }
-    if (!eng->list_need) {
-        int rc;
-        if ((rc = dalloc(eng, &eng->list_need, 1))) return rc;
-        CK(cudaMemsetAsync(eng->list_need, 0, sizeof(int), eng->stream));
-        CK(cudaMallocHost((void **)&eng->list_need_host, sizeof(int)));
-        *eng->list_need_host = 0;
-        CK(cudaEventCreateWithFlags(&eng->ev_need, cudaEventDisableTiming));
-    }
-    if (!eng->lists_on || relaid) {
-        eng->list_k = capped_list_k(eng, std::max(eng->list_k, estimate_list_k(eng)));
-        int rc = alloc_lists(eng);
-        if (rc) return rc;
-        eng->lists_on = true;
-        eng->gen++;
-    }
-    if (eng->split != 1) {   // lists are kept per home cell
-        eng->split = 1;
-        eng->gen++;
-    }
-    return TFG_OK;
-}
-
-int check_lists(tfg_engine *eng) {
-    if (!eng->lists_on || !eng->need_pending) return TFG_OK;
-    const cudaError_t e = cudaEventQuery(eng->ev_need);
-    if (e == cudaErrorNotReady) {
-        cudaGetLastError();
-        return TFG_OK;
-    }
-    CK(e);
-    eng->need_pending = false;
-    const int need = *eng->list_need_host;
-    const int grown = capped_list_k(eng, ((int)(need * 1.25) + 127) & ~127);
-    if (need <= eng->list_k || grown <= eng->list_k) return TFG_OK;
-    // lists that did not fit are evaluated with candidate tests until the next rebuild
-    eng->list_k = grown;
-    int rc = alloc_lists(eng);
-    if (rc) return rc;
-    eng->gen++;
     return TFG_OK;
 }
 
@@ -861,11 +806,15 @@ PairKernelArgs pair_args(tfg_engine *eng) {
     a.pforce = A.pforce;
     a.cell = A.cell;
     a.start = eng->start;
+    a.items = eng->items;
+    a.nitems = reinterpret_cast<const int *>(eng->counters + 1);
+    a.counter = eng->counters + 2;
     a.sval = A.sval;
     a.sq = A.sq;
     a.cap = eng->cap;
     a.force = eng->force;
     a.pots = eng->pots;
+    a.potc = eng->potc;
     a.blob = eng->blob;
     a.blob_floats = eng->blob_floats;
     a.fluxes = eng->fluxes;
@@ -878,25 +827,10 @@ PairKernelArgs pair_args(tfg_engine *eng) {
     a.has_dpd = eng->has_dpd;
     a.flux_sub = -1;
     a.has_flux = eng->has_flux;
-    if (eng->lists_on) {
-        a.vlist = eng->vlist;
-        a.vlen = eng->vlen;
-        a.list_k = eng->list_k;
-        a.list_need = eng->list_need;
-    }
     return a;
 }
 
-const TilePlan &tile_plan(tfg_engine *eng, int split) {
-    if (eng->plan_gen != eng->gen || eng->plan_split != split) {
-        eng->plan = plan_pair_tile((int)eng->order.size(), eng->max_type, eng->blob_floats);
-        eng->plan_gen = eng->gen;
-        eng->plan_split = split;
-    }
-    return eng->plan;
-}
-
-// The tiled half-shell kernel handles at most one species; more go to the stencil kernel.
+// Deterministic mode runs the stencil kernel instead of the tiled one.
 bool use_tile(const tfg_engine *eng) { return !eng->deterministic; }
 
 int force_pass(tfg_engine *eng, bool bonded, bool timed) {
@@ -905,8 +839,7 @@ int force_pass(tfg_engine *eng, bool bonded, bool timed) {
     PairKernelArgs a = pair_args(eng);
     if (eng->n > 0) {
         if (use_tile(eng))
-            launch_pair_tile(a, tile_plan(eng, eng->split), eng->overflow_list, eng->overflow_count, eng->sms, false,
-                             tune_of(eng), s);
+            launch_pair_tile(a, eng->sms, false, tune_of(eng), s);
         else launch_pair(a, s);
     }
     if (timed) launch_stamp(eng->stamps, 2, s);
@@ -929,7 +862,7 @@ int flux_substeps(tfg_engine *eng) {
     for (int sub = 0; sub < eng->max_fluxsteps - 1; sub++) {
         PairKernelArgs a = pair_args(eng);
         a.flux_sub = sub;
-        launch_pair_fluxonly(a, tile_plan(eng, 1), eng->overflow_list, eng->overflow_count, eng->sms, use_tile(eng), s);
+        launch_pair_fluxonly(a, eng->sms, use_tile(eng), s);
         ParticleArrays &A = eng->A[eng->cur];
         launch_flux_integrate(eng->n, eng->cap, eng->nspec, sub, eng->sims_dev, eng->cell_sim, A.cell, A.sval, A.sq,
                               eng->species_flags, s);
@@ -939,8 +872,6 @@ int flux_substeps(tfg_engine *eng) {
 
 int enqueue_step(tfg_engine *eng, bool advance, bool timed) {
     cudaStream_t s = eng->stream;
-    const int nsims = (int)eng->order.size();
-    launch_tick(nsims, eng->sims_dev, eng->red, s);   // also clears the advancing simulations' totals
     if (timed) launch_stamp(eng->stamps, 0, s);
     int rc = bin(eng, 1);
     if (rc) return rc;
@@ -1027,9 +958,8 @@ int run_steps(tfg_engine *eng, int nsteps) {
     // After any change of the captured launch arguments one step runs eagerly (it also sets
     // every kernel's launch attributes up); the others replay the captured step of the
     // current buffer parity.  With phase timing on, every step writes its phase stamps.
-    int rc = check_lists(eng);
-    if (rc) return rc;
     for (int k = 0; k < nsteps; k++) {
+        int rc;
         if (eng->use_graphs && eng->eager_gen == eng->gen) {
             rc = graph_step(eng);
         } else {
@@ -1037,11 +967,6 @@ int run_steps(tfg_engine *eng, int nsteps) {
             eng->eager_gen = eng->gen;
         }
         if (rc) return rc;
-    }
-    if (eng->lists_on && !eng->need_pending) {
-        CK(cudaMemcpyAsync(eng->list_need_host, eng->list_need, sizeof(int), cudaMemcpyDeviceToHost, eng->stream));
-        CK(cudaEventRecord(eng->ev_need, eng->stream));
-        eng->need_pending = true;
     }
     return TFG_OK;
 }
@@ -1059,7 +984,7 @@ int tune_if_needed(tfg_engine *eng) {
 }
 
 int autotune(tfg_engine *eng, bool splits_only) {
-    if (!use_tile(eng) || eng->n == 0 || eng->lists_on) {
+    if (!use_tile(eng) || eng->n == 0) {
         eng->split = 1;
         eng->tune_auto = true;
         eng->tuned_n = eng->n;
@@ -1071,35 +996,28 @@ int autotune(tfg_engine *eng, bool splits_only) {
     int rc = dalloc(eng, &save, nq);
     if (rc) return rc;
     CK(cudaMemcpyAsync(save, eng->A[eng->cur].sq, sizeof(float) * nq, cudaMemcpyDeviceToDevice, s));
-    // candidates: every work split of the tiled kernel with 1, 2 or 4 items per grab, in CTAs
-    // of 8 warps and, for the table variants, of 4; and the home-outer kernel
+    // candidates: every work split of the tiled kernel, in CTAs of 8 warps and, for the table
+    // variants, of 4 (the kernel sizes its grabs itself, so these stay at one item at least)
     const PairKernelArgs a0 = pair_args(eng);
     const bool table_only = !a0.has_dpd && !(a0.nspec > 0 && a0.has_flux);
     std::vector<TileTune> cand;
     for (int split : {1, 2, 7, 14})
-        for (int warps : {8, 4})
-            for (int grab : {1, 2, 4}) {
-                if (warps == 4 && !table_only) continue;
-                // a re-tune keeps the CTA shape and grab and times the splits only
-                if (splits_only && (warps != eng->tune_warps || grab != eng->tune_grab)) continue;
-                TileTune t;
-                t.split = split;
-                t.warps = warps;
-                t.grab = grab;
-                cand.push_back(t);
-            }
-    if (!splits_only && pair_home_eligible(a0)) {
-        TileTune t;
-        t.split = TFG_PAIR_HOME_OUTER;
-        cand.push_back(t);
-    }
+        for (int warps : {8, 4}) {
+            if (warps == 4 && !table_only) continue;
+            // a re-tune keeps the CTA shape and times the splits only
+            if (splits_only && warps != eng->tune_warps) continue;
+            TileTune t;
+            t.split = split;
+            t.warps = warps;
+            cand.push_back(t);
+        }
     // one timed launch of a candidate on freshly initialised forces (ms, or < 0 on error)
     auto trial = [&](const TileTune &tc) -> float {
         rc = bin(eng, 0);
         if (rc) return -1.f;
         PairKernelArgs a = pair_args(eng);
         cudaEventRecord(eng->ev[0], s);
-        launch_pair_tile(a, tile_plan(eng, tc.split), eng->overflow_list, eng->overflow_count, eng->sms, false, tc, s);
+        launch_pair_tile(a, eng->sms, false, tc, s);
         cudaEventRecord(eng->ev[1], s);
         const cudaError_t e = cudaEventSynchronize(eng->ev[1]);
         if (e != cudaSuccess) {
@@ -1236,16 +1154,14 @@ void destroy(tfg_engine *eng) {
     if (eng->stream) cudaStreamSynchronize(eng->stream);
     drop_graphs(eng);
     for (int b = 0; b < 2; b++) free_particles(eng->A[b]);
-    void *bufs[] = {eng->wpots, eng->stamps, eng->force, eng->count, eng->start, eng->lidx, eng->tmp_id, eng->tmp_src, eng->dest,
-                    eng->slot_of_id, eng->scan_sums, eng->cell_sim, eng->overflow_list, eng->overflow_count,
-                    eng->sims_dev, eng->corig, eng->pots, eng->blob, eng->fluxes, eng->rforce, eng->type_mass,
+    void *bufs[] = {eng->wpots, eng->stamps, eng->force, eng->count, eng->start, eng->lidx, eng->bin_tmp, eng->items,
+                    eng->slot_of_id, eng->scan_part, eng->scan_pre, eng->counters, eng->cell_sim,
+                    eng->sims_dev, eng->corig, eng->pots, eng->potc, eng->blob, eng->fluxes, eng->rforce, eng->type_mass,
                     eng->type_dyn, eng->species_flags, eng->bonds, eng->bond_slot, eng->angles, eng->bpots,
-                    eng->bblob, eng->red, eng->err, eng->oldx, eng->vlist, eng->vlen, eng->list_need};
+                    eng->bblob, eng->red, eng->err, eng->oldx};
     for (void *p : bufs) cudaFree(p);
     for (int k = 0; k < 5; k++)
         if (eng->ev[k]) cudaEventDestroy(eng->ev[k]);
-    if (eng->ev_need) cudaEventDestroy(eng->ev_need);
-    if (eng->list_need_host) cudaFreeHost(eng->list_need_host);
     if (eng->own_stream && eng->stream) cudaStreamDestroy(eng->stream);
     delete eng;
 }

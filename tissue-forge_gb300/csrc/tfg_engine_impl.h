@@ -58,26 +58,22 @@ struct tfg_engine {
     float4 *force = nullptr;
     float4 *oldx = nullptr;          // Verlet reference positions by slot
     int oldx_cap = 0;
-    // Verlet pair lists of the tiled pass (table variants): list_k entries per home cell
-    bool lists_wanted = true;        // tfg_set_pair_lists
-    bool lists_on = false;
-    uint32_t *vlist = nullptr;
-    int32_t *vlen = nullptr;
-    size_t vlist_cap = 0, vlen_cap = 0;
-    int list_k = 0;
-    int *list_need = nullptr;        // device: largest list a build asked for
-    int *list_need_host = nullptr;   // pinned copy, read once its event has completed
-    cudaEvent_t ev_need = nullptr;
-    bool need_pending = false;
-    int32_t *count = nullptr, *start = nullptr, *lidx = nullptr, *tmp_id = nullptr, *tmp_src = nullptr,
-            *dest = nullptr, *slot_of_id = nullptr, *scan_sums = nullptr, *cell_sim = nullptr;
-    int *overflow_list = nullptr, *overflow_count = nullptr;
+    int32_t *count = nullptr, *start = nullptr, *lidx = nullptr, *slot_of_id = nullptr, *cell_sim = nullptr;
+    int2 *bin_tmp = nullptr, *items = nullptr;
+    unsigned long long *scan_part = nullptr, *scan_pre = nullptr;
+    size_t items_cap = 0;
+    // device counters: [0] scan ticket, [1] work items of the tiled pair pass, [2] its work
+    // counter, [3] its finished blocks (each returns to zero by itself, but [1])
+    unsigned *counters = nullptr;
+    bool has_ext = false, has_rand = false;   // a force_i or a random force was ever set
     tfg::SimParams *sims_dev = nullptr;
     int sims_cap = 0;
     float *corig = nullptr;
     size_t corig_cap = 0;
     tfg::PotDev *pots = nullptr;
     size_t pots_cap = 0;
+    tfg::PotPair *potc = nullptr;     // the same in the tiled pair pass's compact form
+    size_t potc_cap = 0;
     float *blob = nullptr;
     size_t blob_cap = 0;
     int blob_floats = 0;
@@ -125,10 +121,6 @@ struct tfg_engine {
     int tune_grab = 1;               // tiled pair pass: work items per grab
     bool deterministic = false;      // pair pass without atomics (stencil kernel): reproducible bits
     int capacity_hint = 0;
-    // tiled-pass staging plan, cached for (generation, split)
-    tfg::TilePlan plan;
-    uint64_t plan_gen = 0;
-    int plan_split = 0;
     // CUDA graphs of one step, one per starting buffer parity (a step swaps the particle
     // buffers).  `gen` changes whenever a captured launch argument may have changed
     // (layout, tables, split, stream); a graph captured under another generation is
@@ -181,10 +173,7 @@ inline TileTune tune_of(const tfg_engine *eng) {
     t.grab = eng->tune_grab;
     return t;
 }
-int prepare_lists(tfg_engine *eng, bool relaid);  // allocate / invalidate the Verlet pair lists
-int check_lists(tfg_engine *eng);                 // grow them when a build asked for more
 PairKernelArgs pair_args(tfg_engine *eng);
-const TilePlan &tile_plan(tfg_engine *eng, int split);
 bool use_tile(const tfg_engine *eng);
 PotDev to_dev(const tfg_potential *p);
 int load_sim(tfg_engine *eng, int sim, int n, const float *xg, const int32_t *cellv, const float *xrel,

@@ -53,11 +53,15 @@ struct PairKernelArgs {
     const float4 *pforce;
     const int32_t *cell;
     const int32_t *start;       // ncells+1
+    const int2 *items;          // work items of the tiled pass: (cell, first of up to 32 home particles)
+    const int *nitems;
+    unsigned *counter;          // work counter of the tiled pass and its finished blocks
     const float *sval;
     float *sq;
     int cap;
     float4 *force;              // out: f.xyz, number density
     const PotDev *pots;         // nsims * max_type^2
+    const PotPair *potc;        // the same, compact (tiled pass)
     const float *blob;
     int blob_floats;
     const PotDev *wpots;        // nsims * 6 * max_type wall potentials
@@ -76,60 +80,27 @@ struct PairKernelArgs {
                                 // nr_fluxsteps - 1 > flux_sub take part); -1: the full pass
     bool has_dpd;               // any type pair uses a DPD potential
     bool has_flux;              // any type pair has fluxes
-    // Verlet pair lists (tiled pass, table potentials): per home cell, the staged-index
-    // pairs (i | k << 16) within the list radius found at the simulation's last rebuild,
-    // one kListEnd marker after each staging chunk, in interleaved groups of 128
-    uint32_t *vlist;            // list_k entries per home cell (a multiple of 128)
-    int32_t *vlen;              // entries of each home cell's list; -1: none (candidate tests)
-    int list_k;
-    int *list_need;             // largest list a build asked for (atomicMax)
 };
-
-constexpr uint32_t kListEnd = 0xffffffffu;
 
 // Full-stencil kernel: one thread per particle, no atomics.  General path (any number
 // of species); force[] must hold the initial force (external + random, density W(0)).
 void launch_pair(const PairKernelArgs &a, cudaStream_t s);
-// Tiled half-shell kernel (one species at most) plus its overflow pass; force[] must hold
-// the initial force, to which both partners' contributions are added atomically.
-// `split` = warps per home cell (1, 2, 7 or 14): the cell's 14 tasks are divided into
-// that many work items.
-// Shared-memory staging of the tiled pass: every potential table and descriptor of the
-// arena is staged per CTA when they fit (the usual case for one simulation), else none is
-// and they are read through L1.
-struct TilePlan {
-    int stage_floats = 0;
-    int stage_pots = 0;
-};
-TilePlan plan_pair_tile(int nsims, int max_type, int blob_floats);
 // Launch configuration of the nonbonded pass, picked by the autotuner: the work split (warps
-// per home cell: 1, 2, 7 or 14, or TFG_PAIR_HOME_OUTER for the home-outer kernel), the
-// warps per CTA of the tiled kernel's table variants (8, or 4 with twice the CTAs per SM),
-// and the work items a warp takes from the shared counter at a time.
+// per home cell: 1, 2, 7 or 14; the cell's 14 tasks are divided into that many work items;
+// TFG_PAIR_HOME_OUTER means 1), the warps per CTA of the table variants (8, or 4 with twice
+// the CTAs per SM), and the fewest work items a warp takes from the shared counter at a time.
 struct TileTune {
     int split = 1;
     int warps = 8;
     int grab = 1;
 };
-void launch_pair_tile(const PairKernelArgs &a, const TilePlan &plan, int *overflow_list, int *overflow_count, int sms,
-                      bool signature, const TileTune &tune, cudaStream_t s);
-// Overflow pass of the tiled kernels' table variant: the home cells listed in
-// overflow_list[0 .. overflow_count[0]), one warp each, global-memory candidates and atomics.
-void launch_pair_overflow(const PairKernelArgs &a, int *overflow_list, int *overflow_count, bool signature, int sms,
-                          cudaStream_t s);
-// Home-particle-outer pass (split TFG_PAIR_HOME_OUTER): tabulated potentials only, no DPD,
-// fluxes or Verlet pair lists.  overflow_count must be zeroed before the launch.
-void launch_pair_home(const PairKernelArgs &a, int *overflow_list, int *overflow_count, int sms, bool signature,
-                      cudaStream_t s);
-inline bool pair_home_eligible(const PairKernelArgs &a) {
-    return !a.has_dpd && !(a.nspec > 0 && a.has_flux) && !a.vlist && a.flux_sub < 0;
-}
-int pair_tile_capacity();
+// Tiled half-shell kernel; force[] must hold the initial force, to which both partners'
+// contributions are added atomically.
+void launch_pair_tile(const PairKernelArgs &a, int sms, bool signature, const TileTune &tune, cudaStream_t s);
 void launch_pair_stencil_fluxonly(const PairKernelArgs &a, cudaStream_t s);
 // Flux-only substep pass (a.flux_sub >= 0): species flux increments of the pair set, no
 // forces, densities or energies (runner_dopair_fluxonly / runner_doself_fluxonly).
-void launch_pair_fluxonly(const PairKernelArgs &a, const TilePlan &plan, int *overflow_list, int *overflow_count,
-                          int sms, bool tile, cudaStream_t s);
+void launch_pair_fluxonly(const PairKernelArgs &a, int sms, bool tile, cudaStream_t s);
 // Same stencil walk and pair decision as launch_pair, writing only the per-particle
 // pair signature (used to prove the pair set bit-exact against the oracle).
 void launch_pair_signature(const PairKernelArgs &a, cudaStream_t s);

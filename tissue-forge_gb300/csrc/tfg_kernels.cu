@@ -104,17 +104,17 @@ __global__ void k_stamp(unsigned long long *t, int k) {
     t[k] = v;
 }
 
-// time += 1 (engine_step, tfEngine.cpp:1387) and, in Verlet mode, the rebuild decision of
-// engine_verlet_update (tfEngine.cpp:234-290): rebuild when 2 * maxdx > skin, maxdx being
-// the largest displacement since the last rebuild, measured after the previous advance.
-// One step's start for every simulation: stop it if it has reached its stop time, else
-// advance its clock and clear its FP64 totals (a stopped simulation keeps the totals of its
-// last step).
-__global__ void k_tick(int nsims, SimParams *sims, double *red) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nsims) return;
-    SimParams &P = sims[k];
-    if (P.stop_at >= 0 && P.time >= P.stop_at) {
+// One step's start for a simulation: stop it if it has reached its stop time, else advance its
+// clock (time += 1, engine_step, tfEngine.cpp:1387) and clear its FP64 totals (a stopped
+// simulation keeps the totals of its last step).  In Verlet mode, the rebuild decision of
+// engine_verlet_update (tfEngine.cpp:234-290): rebuild when 2 * maxdx > skin, maxdx being the
+// largest displacement since the last rebuild, measured after the previous advance.
+__device__ __forceinline__ bool stops_now(const SimParams &P) { return P.stop_at >= 0 && P.time >= P.stop_at; }
+__device__ __forceinline__ bool rebuilds_now(const SimParams &P) {
+    return P.verlet_rebuild == 2 || __fmul_rn(2.0f, __fsqrt_rn(__uint_as_float(P.verlet_maxdx2))) > P.skin;
+}
+__device__ __forceinline__ void tick(SimParams &P, double *red) {
+    if (stops_now(P)) {
         P.stopped = 1;
         if (P.verlet_rebuild == 1) P.verlet_rebuild = 0;
         return;
@@ -123,13 +123,8 @@ __global__ void k_tick(int nsims, SimParams *sims, double *red) {
     P.time += 1;
     for (int r = 0; r < RED_COUNT; r++) red[P.red_base + r] = 0.0;
     if (P.flags & TFG_ENGINE_VERLET) {
-        int rb = P.verlet_rebuild == 2;
-        float m = 0.f;
-        if (!rb) {
-            m = __fsqrt_rn(__uint_as_float(P.verlet_maxdx2));
-            rb = __fmul_rn(2.0f, m) > P.skin;
-        }
-        P.verlet_maxdx = rb ? 0.f : m;
+        const bool rb = rebuilds_now(P);
+        P.verlet_maxdx = rb ? 0.f : __fsqrt_rn(__uint_as_float(P.verlet_maxdx2));
         P.verlet_rebuild = rb;
         P.verlet_maxdx2 = 0u;
         if (rb) P.verlet_rebuilds += 1;
@@ -186,7 +181,17 @@ __global__ void k_relocate(int n, int src0, int dst0, int cap_src, int cap_dst, 
     }
 }
 
-// Re-check of the cell-relative position (space_shuffle_local) and per-cell counting.
+// Binning, in four launches.  It is bound by launches and L2 latency below about 100,000
+// particles and by HBM above:
+//   k_bin_count    re-check of the cell-relative positions, count per cell
+//   k_scan         block-local scan of the counts; the last block to finish scans the block
+//                  totals; the simulations' tick
+//   k_place        final cell starts, the pair pass's work items, (id, slot) into cell order
+//   k_rank_scatter rank by id inside the cell, then the state itself, with the force init
+
+// Re-check of the cell-relative position (space_shuffle_local) and per-cell counting.  The
+// simulations' clocks advance in the next kernel, so their decisions for this step are
+// taken from the state before it.
 __global__ void k_bin_count(int n, const SimParams *sims, const int32_t *cell_sim, float4 *pos, int32_t *cell,
                             int32_t *count, int32_t *lidx, int shuffle) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -196,7 +201,7 @@ __global__ void k_bin_count(int n, const SimParams *sims, const int32_t *cell_si
         const SimParams &P = sims[cell_sim[c]];
         // Verlet mode re-bins only on rebuild steps (engine_verlet_update -> engine_shuffle);
         // a stopped simulation stays as it is
-        if (P.stopped || ((P.flags & TFG_ENGINE_VERLET) && !P.verlet_rebuild)) {
+        if (stops_now(P) || ((P.flags & TFG_ENGINE_VERLET) && !rebuilds_now(P))) {
             lidx[i] = atomicAdd(&count[c], 1);
             return;
         }
@@ -219,141 +224,162 @@ __global__ void k_bin_count(int n, const SimParams *sims, const int32_t *cell_si
     lidx[i] = atomicAdd(&count[c], 1);
 }
 
-__device__ __forceinline__ int block_exclusive_scan(int v, int *tot) {
-    __shared__ int ws[32];
+constexpr int kScanThreads = 1024, kScanCells = 4 * kScanThreads;   // cells per block
+
+// Exclusive block scan of (particles, items), packed as low and high word.
+__device__ __forceinline__ unsigned long long block_scan2(unsigned long long v, unsigned long long *tot) {
+    __shared__ unsigned long long ws[32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    int x = v;
+    unsigned long long x = v;
     for (int o = 1; o < 32; o <<= 1) {
-        int y = __shfl_up_sync(0xffffffffu, x, o);
+        const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
         if (lane >= o) x += y;
     }
     if (lane == 31) ws[w] = x;
     __syncthreads();
     if (w == 0) {
-        int s = lane < (int)(blockDim.x >> 5) ? ws[lane] : 0;
+        unsigned long long s = lane < (int)(blockDim.x >> 5) ? ws[lane] : 0;
         for (int o = 1; o < 32; o <<= 1) {
-            int y = __shfl_up_sync(0xffffffffu, s, o);
+            const unsigned long long y = __shfl_up_sync(0xffffffffu, s, o);
             if (lane >= o) s += y;
         }
         ws[lane] = s;
     }
     __syncthreads();
-    int excl = x - v + (w > 0 ? ws[w - 1] : 0);
-    if (tot) *tot = ws[(blockDim.x >> 5) - 1];
+    const unsigned long long excl = x - v + (w > 0 ? ws[w - 1] : 0);
+    *tot = ws[(blockDim.x >> 5) - 1];
     __syncthreads();
     return excl;
 }
 
-__global__ void k_scan_local(const int32_t *count, int n, int32_t *start, int32_t *sums) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    int tot;
-    int ex = block_exclusive_scan(i < n ? count[i] : 0, &tot);
-    if (i < n) start[i] = ex;
-    if (threadIdx.x == 0) sums[blockIdx.x] = tot;
-}
+// Work items of a cell with n particles: one per 32 home particles.
+__device__ __forceinline__ int cell_items(int n) { return (n + 31) >> 5; }
 
-__global__ void k_scan_sums(int32_t *sums, int nb) {
-    const int per = (nb + blockDim.x - 1) / blockDim.x;
-    const int b0 = threadIdx.x * per;
-    int local = 0;
-    for (int k = 0; k < per; k++) if (b0 + k < nb) local += sums[b0 + k];
-    int run = block_exclusive_scan(local, nullptr);
+// part[c]: particles and items of the block's cells before c; pre[b]: of the blocks before b,
+// pre[number of blocks]: all.  The counts are cleared for the next binning.
+__global__ void __launch_bounds__(kScanThreads) k_scan(int ncells, int32_t *count, unsigned long long *part,
+                                                       unsigned long long *pre, unsigned *ticket, int do_tick,
+                                                       int nsims, SimParams *sims, double *red) {
+    if (do_tick)
+        for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nsims; k += gridDim.x * blockDim.x) tick(sims[k], red);
+    const int c = blockIdx.x * kScanCells + 4 * threadIdx.x;
+    int m[4];
+    unsigned long long v = 0;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        m[k] = c + k < ncells ? count[c + k] : 0;
+        v += (unsigned long long)cell_items(m[k]) << 32 | (unsigned)m[k];
+    }
+    unsigned long long tot, ex = block_scan2(v, &tot);
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        if (c + k < ncells) {
+            part[c + k] = ex;
+            if (m[k]) count[c + k] = 0;
+            ex += (unsigned long long)cell_items(m[k]) << 32 | (unsigned)m[k];
+        }
+    __shared__ bool last;
+    if (threadIdx.x == 0) {
+        pre[blockIdx.x] = tot;
+        __threadfence();
+        last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    // the last block to finish turns the block totals into prefixes
+    const int nb = gridDim.x, per = (nb + kScanThreads - 1) / kScanThreads, b0 = threadIdx.x * per;
+    unsigned long long sum = 0;
+    for (int k = 0; k < per; k++)
+        if (b0 + k < nb) sum += __ldcg(&pre[b0 + k]);
+    unsigned long long all, run = block_scan2(sum, &all);
     for (int k = 0; k < per; k++)
         if (b0 + k < nb) {
-            int s = sums[b0 + k];
-            sums[b0 + k] = run;
-            run += s;
+            const unsigned long long t = __ldcg(&pre[b0 + k]);
+            pre[b0 + k] = run;
+            run += t;
         }
+    if (threadIdx.x == 0) pre[nb] = all;
 }
 
-__global__ void k_scan_add(int32_t *start, const int32_t *sums, const int32_t *count, int n) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void k_place(int n, int ncells, const int32_t *cell, const int32_t *lidx, const unsigned long long *part,
+                        const unsigned long long *pre, int nb, const float4 *aux, int32_t *start, int2 *items,
+                        int *nitems, int2 *tmp) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < ncells) {
+        const unsigned long long a = part[i] + pre[i / kScanCells];
+        const unsigned long long b = i + 1 < ncells ? part[i + 1] + pre[(i + 1) / kScanCells] : pre[nb];
+        start[i] = (int)(unsigned)a;
+        const int i0 = (int)(a >> 32), i1 = (int)(b >> 32);
+        for (int k = i0; k < i1; k++) items[k] = make_int2(i, 32 * (k - i0));
+        if (i == ncells - 1) {
+            start[ncells] = (int)(unsigned)b;
+            *nitems = i1;
+        }
+    }
     if (i < n) {
-        int s = start[i] + sums[blockIdx.x];
-        start[i] = s;
-        if (i == n - 1) start[n] = s + count[i];
+        const int c = cell[i];
+        const int p = (int)(unsigned)(part[c] + pre[c / kScanCells]) + lidx[i];
+        tmp[p] = make_int2(__float_as_int(aux[i].w), i);
     }
 }
 
-__global__ void k_place(int n, const int32_t *cell, const int32_t *lidx, const int32_t *start, const float4 *aux,
-                        int32_t *tmp_id, int32_t *tmp_src) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int p = start[cell[i]] + lidx[i];
-    tmp_id[p] = __float_as_int(aux[i].w);
-    tmp_src[p] = i;
-}
-
-// Deterministic order inside a cell: rank by particle id (one warp per cell).  Cells of
-// up to 32 particles rank in registers; larger cells compare against global memory.
-__global__ void k_rank(int ncells, const int32_t *start, const int32_t *tmp_id, const int32_t *tmp_src,
-                       int32_t *dest) {
-    int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
-    if (w >= ncells) return;
-    int s0 = start[w], s1 = start[w + 1];
-    const int n = s1 - s0;
-    if (n == 0) return;
-    if (n <= 32) {
-        const int my = lane < n ? tmp_id[s0 + lane] : 0x7fffffff;
-        int r = 0;
-        for (int o = 0; o < n; o++) r += __shfl_sync(0xffffffffu, my, o) < my;
-        if (lane < n) dest[tmp_src[s0 + lane]] = s0 + r;
-        return;
-    }
-    for (int e = s0 + lane; e < s1; e += 32) {
-        int my = tmp_id[e];
-        int r = 0;
-        for (int o = s0; o < s1; o++) r += tmp_id[o] < my;
-        dest[tmp_src[e]] = s0 + r;
-    }
-}
-
-__global__ void k_scatter(int n, int cap, int nspec, const int32_t *dest, ParticleArrays src, ParticleArrays dst,
-                          int32_t *slot_of_id, const SimParams *sims, const int32_t *cell_sim, const float4 *rforce,
-                          float4 *force, float4 *oldx) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int d = dest[i];
-    const float4 ax = src.aux[i];
-    const float4 p = src.pos[i];
-    const float4 fe = src.fext[i];
+// One thread per place p of the cell order: its particle's rank by id among the cell's (the
+// deterministic order inside a cell) gives the slot its state moves to.  kExt: some simulation
+// has external forces; kRand: some type has had a random force (its persistent value moves).
+template <bool kExt, bool kRand>
+__global__ void k_rank_scatter(int n, int cap, int nspec, const int2 *__restrict__ tmp, const int32_t *__restrict__ start,
+                               ParticleArrays src, ParticleArrays dst, int32_t *slot_of_id, const SimParams *sims,
+                               const int32_t *cell_sim, const float4 *rforce, float4 *force, float4 *oldx) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const int2 me = tmp[t];
+    const int id = me.x, i = me.y;
     const int c = src.cell[i];
-    float4 pf = src.pforce[i];
-    const int id = __float_as_int(ax.w);
+    const float4 ax = src.aux[i], p = src.pos[i], v = src.vel[i];
+    const int s0 = start[c], s1 = start[c + 1];
     const SimParams &P = sims[cell_sim[c]];
-    const float4 rf = rforce[P.type_base + __float_as_int(p.w)];
-    if (rf.w != 0.f) {
+    int d = s0;
+    for (int o = s0; o < s1; o++) d += tmp[o].x < id;
+    float4 fe = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (kExt) {
+        fe = src.fext[i];
+        dst.fext[d] = fe;
+    }
+    if (kRand) {
+        const float4 rf = rforce[P.type_base + __float_as_int(p.w)];
         const int lid = id - P.id_off;
-        const int dur = (int)rf.z;
-        if ((P.time + lid) % dur == 0) {
+        float4 pf;
+        if (rf.w != 0.f && (P.time + lid) % (int)rf.z == 0) {
             U4 r = philox({(uint32_t)P.time, (uint32_t)lid, 0u, STREAM_FORCE}, (uint32_t)P.seed,
                           (uint32_t)(P.seed >> 32));
             const float theta = 6.283185307179586f * u01(r.x);
             const float phi = acosf(1.f - 2.f * u01(r.y));
             const float g = sqrtf(-2.0f * logf(u01(r.z))) * cosf(6.283185307179586f * u01(r.w));
             const float rr = rf.x + rf.y * g;
-            pf.x = rr * sinf(phi) * cosf(theta);
-            pf.y = rr * sinf(phi) * sinf(theta);
-            pf.z = rr * cosf(phi);
+            pf = make_float4(rr * sinf(phi) * cosf(theta), rr * sinf(phi) * sinf(theta), rr * cosf(phi), 0.f);
+        } else {
+            pf = src.pforce[i];
         }
-        force[d] = make_float4(fe.x + pf.x, fe.y + pf.y, fe.z + pf.z, P.self_density);
-    } else {
-        force[d] = make_float4(fe.x, fe.y, fe.z, P.self_density);
+        dst.pforce[d] = pf;
+        if (rf.w != 0.f) {
+            fe.x += pf.x;
+            fe.y += pf.y;
+            fe.z += pf.z;
+        }
     }
+    force[d] = make_float4(fe.x, fe.y, fe.z, P.self_density);
     dst.pos[d] = p;
     // Verlet reference positions, stored after the rebuild's re-binning (tfEngine.cpp:308-335)
     if (oldx && (P.flags & TFG_ENGINE_VERLET) && P.verlet_rebuild) oldx[d] = make_float4(p.x, p.y, p.z, 0.f);
-    dst.vel[d] = src.vel[i];
+    dst.vel[d] = v;
     dst.aux[d] = ax;
-    dst.fext[d] = fe;
-    dst.pforce[d] = pf;
     dst.cell[d] = c;
     for (int s = 0; s < nspec; s++) {
         dst.sval[s * cap + d] = src.sval[s * cap + i];
         dst.sq[s * cap + d] = src.sq[s * cap + i];
     }
-    slot_of_id[id] = d;
+    if (slot_of_id) slot_of_id[id] = d;
 }
 
 // bond_eval (tfBond.cpp:97-345) for table potentials; one thread per bond.
@@ -708,10 +734,6 @@ inline int nblk(long long n, int t) { return (int)((n + t - 1) / t); }
 
 void launch_stamp(unsigned long long *t, int k, cudaStream_t s) { k_stamp<<<1, 1, 0, s>>>(t, k); }
 
-void launch_tick(int nsims, SimParams *sims, double *red, cudaStream_t s) {
-    if (nsims > 0) k_tick<<<nblk(nsims, 128), 128, 0, s>>>(nsims, sims, red);
-}
-
 void launch_setpartp(int n, const float *xg, const SimParams &P, float3 lo, float3 hi, float3 org, float3 ih,
                      int slot0, int32_t *cell, float4 *pos, float4 *aux, const int32_t *type, uint32_t *err,
                      cudaStream_t s) {
@@ -726,23 +748,26 @@ void launch_relocate(int n, int src0, int dst0, int cap_src, int cap_dst, int ns
                                                           dst);
 }
 
+int scan_blocks(int ncells) { return nblk(ncells, kScanCells); }
+
 void launch_bin(const BinArgs &b, cudaStream_t s) {
-    cudaMemsetAsync(b.count, 0, sizeof(int32_t) * b.ncells, s);
     if (b.n > 0)
         k_bin_count<<<nblk(b.n, kThreads), kThreads, 0, s>>>(b.n, b.sims, b.cell_sim, b.src.pos, b.src.cell, b.count,
                                                             b.lidx, b.shuffle);
-    const int nbs = nblk(b.ncells, 1024);
-    k_scan_local<<<nbs, 1024, 0, s>>>(b.count, b.ncells, b.start, b.scan_sums);
-    k_scan_sums<<<1, 1024, 0, s>>>(b.scan_sums, nbs);
-    k_scan_add<<<nbs, 1024, 0, s>>>(b.start, b.scan_sums, b.count, b.ncells);
-    if (b.n > 0) {
-        k_place<<<nblk(b.n, kThreads), kThreads, 0, s>>>(b.n, b.src.cell, b.lidx, b.start, b.src.aux, b.tmp_id,
-                                                        b.tmp_src);
-        k_rank<<<nblk((long long)b.ncells * 32, kThreads), kThreads, 0, s>>>(b.ncells, b.start, b.tmp_id, b.tmp_src,
-                                                                             b.dest);
-        k_scatter<<<nblk(b.n, kThreads), kThreads, 0, s>>>(b.n, b.cap, b.nspec, b.dest, b.src, b.dst, b.slot_of_id,
-                                                          b.sims, b.cell_sim, b.rforce, b.force, b.oldx);
-    }
+    const int nb = scan_blocks(b.ncells);
+    k_scan<<<nb, kScanThreads, 0, s>>>(b.ncells, b.count, b.part, b.pre, b.ticket, b.shuffle, b.nsims, b.sims, b.red);
+    k_place<<<nblk(b.n > b.ncells ? b.n : b.ncells, kThreads), kThreads, 0, s>>>(
+        b.n, b.ncells, b.src.cell, b.lidx, b.part, b.pre, nb, b.src.aux, b.start, b.items, b.nitems, b.tmp);
+    if (b.n <= 0) return;
+    const int g = nblk(b.n, kThreads);
+#define TFG_SCATTER(E, R)                                                                                       \
+    k_rank_scatter<E, R><<<g, kThreads, 0, s>>>(b.n, b.cap, b.nspec, b.tmp, b.start, b.src, b.dst, b.slot_of_id, \
+                                                b.sims, b.cell_sim, b.rforce, b.force, b.oldx)
+    if (b.has_ext && b.has_rand) TFG_SCATTER(true, true);
+    else if (b.has_ext) TFG_SCATTER(true, false);
+    else if (b.has_rand) TFG_SCATTER(false, true);
+    else TFG_SCATTER(false, false);
+#undef TFG_SCATTER
 }
 
 void launch_bonds(int nb, const SimParams *sims, const int32_t *cell_sim, const int2 *bonds, const int32_t *bslot,

@@ -11,17 +11,26 @@ constexpr int kThreads = 256;
 // cell (ranked by particle id inside a cell), scatter from `src` into `dst`, and the
 // force initialisation of the coming pair pass.
 struct BinArgs {
-    int n, cap, ncells, nspec, shuffle;
-    const SimParams *sims;
+    int n, cap, ncells, nspec, nsims;
+    int shuffle;                  // a step's binning: the simulations tick and their particles are re-checked
+    bool has_ext, has_rand;       // external / random forces ever set: fext / pforce move too (else they are zero)
+    SimParams *sims;
+    double *red;
     const int32_t *cell_sim;
     ParticleArrays src, dst;
-    int32_t *count, *start, *lidx, *tmp_id, *tmp_src, *dest, *scan_sums, *slot_of_id;
+    int32_t *count, *start, *lidx;   // count is zero between binnings
+    int32_t *slot_of_id;             // null: no bonds or angles
+    int2 *tmp;                       // (id, slot before) in cell order
+    unsigned long long *part, *pre;  // scan scratch: ncells, scan_blocks(ncells) + 1
+    unsigned *ticket;
+    int2 *items;                     // the pair pass's work: (cell, first of up to 32 home particles)
+    int *nitems;
     const float4 *rforce;
     float4 *force;
     float4 *oldx;   // Verlet reference positions by slot (written on rebuild steps), or null
 };
 
-void launch_tick(int nsims, SimParams *sims, double *red, cudaStream_t s);
+int scan_blocks(int ncells);
 // One thread writes the GPU global timer (ns) into t[k]: phase boundaries of a step, valid
 // inside captured graphs (event timing is not).
 void launch_stamp(unsigned long long *t, int k, cudaStream_t s);
