@@ -150,6 +150,25 @@ __host__ __device__ inline bool on_wall(const SimParams &P, int w, int a, int b,
     return (w & 1) ? l + 1 == P.cdim[ax] : l == 0;
 }
 
+// ---------------- programmatic launch ----------------
+// First statement of every kernel of a step: let the next kernel's blocks start, then wait
+// until the kernel before has finished and its writes are visible.  All threads call it before
+// they touch memory, so a kernel's end implies the end of every kernel before it.
+__device__ __forceinline__ void step_kernel_begin() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// GPU global timer (ns) into *t: the phase boundaries of a step, written by its kernels.
+__device__ __forceinline__ unsigned long long global_timer() {
+    unsigned long long v;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(v));
+    return v;
+}
+__device__ __forceinline__ void stamp_begin(unsigned long long *t) {
+    if (t && blockIdx.x == 0 && threadIdx.x == 0) *t = global_timer();
+}
+
 // ---------------- Philox4x32-10 (Salmon et al., SC'11) ----------------
 struct U4 { uint32_t x, y, z, w; };
 

@@ -259,7 +259,7 @@ int relayout(tfg_engine *eng) {
         CK(cudaMemsetAsync(eng->count, 0, sizeof(int32_t) * cc, s));
         eng->cells_cap = cc;
     }
-    if ((rc = ensure(eng, &eng->items, eng->items_cap, (size_t)C + N / 32 + 1))) return rc;
+    if ((rc = ensure(eng, &eng->items, eng->items_cap, (size_t)C + N / 8 + 1))) return rc;
     CK(cudaMemcpyAsync(eng->cell_sim, cell_sim.data(), sizeof(int32_t) * std::max(C, 1), cudaMemcpyHostToDevice, s));
     if ((int)order.size() > eng->err_slots) {
         const int slots = std::max((int)order.size(), 2 * eng->err_slots);
@@ -739,8 +739,16 @@ int load_sim(tfg_engine *eng, int sim, int n, const float *xg, const int32_t *ce
     return TFG_OK;
 }
 
-int bin(tfg_engine *eng, int shuffle) {
+// Home particles per work item of the tiled pass.  A small arena leaves most warps without an
+// item, and its time is that of the longest one, a crowded cell's: 8 instead of 32 took the
+// pass from 34 to 17 us on 4,000 clustered cells and from 39 to 24 us on 20,000.  More items
+// test more candidates for the same pairs: on 150,001 uniform cells 8, 16 and 32 take 93, 84
+// and 82 us, on 50,000 clustered ones 38, 39 and 46.
+static int log2_homes(const tfg_engine *eng) { return eng->n < 24000 ? 3 : (eng->n < 100000 ? 4 : 5); }
+
+int bin(tfg_engine *eng, int shuffle, bool timed) {
     BinArgs b;
+    b.stamp = timed ? eng->stamps : nullptr;
     b.n = eng->n;
     b.cap = eng->cap;
     b.ncells = eng->ncells;
@@ -759,6 +767,7 @@ int bin(tfg_engine *eng, int shuffle) {
     b.pre = eng->scan_pre;
     b.ticket = eng->counters;
     b.items = eng->items;
+    b.log2_homes = log2_homes(eng);
     b.nitems = reinterpret_cast<int *>(eng->counters + 1);
     b.nsims = (int)eng->order.size();
     b.red = eng->red;
@@ -807,6 +816,7 @@ PairKernelArgs pair_args(tfg_engine *eng) {
     a.cell = A.cell;
     a.start = eng->start;
     a.items = eng->items;
+    a.homes = 1 << log2_homes(eng);
     a.nitems = reinterpret_cast<const int *>(eng->counters + 1);
     a.counter = eng->counters + 2;
     a.sval = A.sval;
@@ -837,19 +847,21 @@ int force_pass(tfg_engine *eng, bool bonded, bool timed) {
     cudaStream_t s = eng->stream;
     ParticleArrays &A = eng->A[eng->cur];
     PairKernelArgs a = pair_args(eng);
+    if (timed && eng->max_fluxsteps <= 1) a.stamp = eng->stamps + 1;   // else stamped before the substeps
     if (eng->n > 0) {
-        if (use_tile(eng))
+        if (use_tile(eng)) {
             launch_pair_tile(a, eng->sms, false, tune_of(eng), s);
-        else launch_pair(a, s);
+        } else {
+            if (a.stamp) launch_stamp(a.stamp, 0, s);
+            launch_pair(a, s);
+        }
     }
-    if (timed) launch_stamp(eng->stamps, 2, s);
     if (bonded) {
         launch_bonds(eng->nb, eng->sims_dev, eng->cell_sim, eng->bonds, eng->bond_slot, eng->bpots, eng->bblob,
-                     eng->slot_of_id, A.pos, A.aux, A.cell, eng->force, eng->red, s);
+                     eng->slot_of_id, A.pos, A.aux, A.cell, eng->force, eng->red, timed ? eng->stamps + 2 : nullptr, s);
         launch_angles(eng->na, eng->sims_dev, eng->cell_sim, eng->angles, eng->bpots, eng->bblob, eng->slot_of_id,
-                      A.pos, A.cell, eng->force, eng->red, s);
+                      A.pos, A.cell, eng->force, eng->red, timed && eng->nb == 0 ? eng->stamps + 2 : nullptr, s);
     }
-    if (timed) launch_stamp(eng->stamps, 3, s);
     return check_launch(eng);
 }
 
@@ -872,17 +884,19 @@ int flux_substeps(tfg_engine *eng) {
 
 int enqueue_step(tfg_engine *eng, bool advance, bool timed) {
     cudaStream_t s = eng->stream;
-    if (timed) launch_stamp(eng->stamps, 0, s);
-    int rc = bin(eng, 1);
+    // the step's kernels stamp the phase boundaries themselves; without particles they do not run
+    if (eng->n == 0 && timed)
+        for (int k = 0; k < 5; k++) launch_stamp(eng->stamps, k, s);
+    int rc = bin(eng, 1, timed);
     if (rc) return rc;
-    if (timed) launch_stamp(eng->stamps, 1, s);
+    if (timed && eng->max_fluxsteps > 1) launch_stamp(eng->stamps, 1, s);
     if ((rc = flux_substeps(eng))) return rc;
     rc = force_pass(eng, true, timed);
     if (rc) return rc;
     if (advance)
         launch_advance(eng->n, eng->cap, eng->nspec, eng->sims_dev, eng->cell_sim, eng->A[eng->cur], eng->force,
-                       eng->type_mass, eng->type_dyn, eng->species_flags, eng->oldx, eng->red, eng->err, s);
-    if (timed) launch_stamp(eng->stamps, 4, s);
+                       eng->type_mass, eng->type_dyn, eng->species_flags, eng->oldx, eng->red, eng->err, eng->stamps,
+                       timed ? 1 << 3 | (eng->nb + eng->na == 0) << 2 : 0, s);
     return check_launch(eng);
 }
 

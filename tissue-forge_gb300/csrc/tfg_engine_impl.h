@@ -155,7 +155,7 @@ int sim_status(tfg_engine *eng, int sim, int *status);
 int sim_check(tfg_engine *eng, int sim);        // TFG_OK when `sim` names a live simulation
 int add_sim(tfg_engine *eng, const tfg_engine_desc *d, int *out);
 int commit(tfg_engine *eng);                    // re-lay the arena out and upload tables when dirty
-int bin(tfg_engine *eng, int shuffle);
+int bin(tfg_engine *eng, int shuffle, bool timed = false);
 int force_pass(tfg_engine *eng, bool bonded, bool timed);
 int one_step(tfg_engine *eng, bool advance, bool timed);
 void advance_clocks(tfg_engine *eng);           // host clocks, by k_tick's rule (stops included)

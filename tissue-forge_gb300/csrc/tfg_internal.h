@@ -24,6 +24,23 @@ struct ParticleArrays {
     float *sq = nullptr;       // flux increments, [s * cap + slot]
 };
 
+// Launch a kernel that begins with step_kernel_begin(): its blocks may be set up while the
+// kernel before it still runs (programmatic dependent launch, in graphs too).
+template <typename... P, typename... A>
+inline void launch_step_kernel(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // Reduction slots in the device double array.
 enum RedSlot : int {
     RED_EPOT_NONBOND = 0,
@@ -53,8 +70,10 @@ struct PairKernelArgs {
     const float4 *pforce;
     const int32_t *cell;
     const int32_t *start;       // ncells+1
-    const int2 *items;          // work items of the tiled pass: (cell, first of up to 32 home particles)
+    const int2 *items;          // work items of the tiled pass: (cell, first of up to `homes` home particles)
     const int *nitems;
+    int homes;                  // 8, 16 or 32
+    unsigned long long *stamp;  // where the pass's begin is stamped, or null
     unsigned *counter;          // work counter of the tiled pass and its finished blocks
     const float *sval;
     float *sq;

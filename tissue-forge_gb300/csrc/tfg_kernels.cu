@@ -99,9 +99,7 @@ __device__ __forceinline__ void keyed_add3(double *red, int rb, int s0, float v0
 }
 
 __global__ void k_stamp(unsigned long long *t, int k) {
-    unsigned long long v;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(v));
-    t[k] = v;
+    t[k] = global_timer();
 }
 
 // One step's start for a simulation: stop it if it has reached its stop time, else advance its
@@ -193,7 +191,9 @@ __global__ void k_relocate(int n, int src0, int dst0, int cap_src, int cap_dst, 
 // simulations' clocks advance in the next kernel, so their decisions for this step are
 // taken from the state before it.
 __global__ void k_bin_count(int n, const SimParams *sims, const int32_t *cell_sim, float4 *pos, int32_t *cell,
-                            int32_t *count, int32_t *lidx, int shuffle) {
+                            int32_t *count, int32_t *lidx, int shuffle, unsigned long long *stamp) {
+    step_kernel_begin();
+    stamp_begin(stamp);
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     int c = cell[i];
@@ -252,14 +252,15 @@ __device__ __forceinline__ unsigned long long block_scan2(unsigned long long v, 
     return excl;
 }
 
-// Work items of a cell with n particles: one per 32 home particles.
-__device__ __forceinline__ int cell_items(int n) { return (n + 31) >> 5; }
+// Work items of a cell with n particles: one per 2^log2_homes home particles.
+__device__ __forceinline__ int cell_items(int n, int log2_homes) { return (n + (1 << log2_homes) - 1) >> log2_homes; }
 
 // part[c]: particles and items of the block's cells before c; pre[b]: of the blocks before b,
 // pre[number of blocks]: all.  The counts are cleared for the next binning.
 __global__ void __launch_bounds__(kScanThreads) k_scan(int ncells, int32_t *count, unsigned long long *part,
-                                                       unsigned long long *pre, unsigned *ticket, int do_tick,
-                                                       int nsims, SimParams *sims, double *red) {
+                                                       unsigned long long *pre, unsigned *ticket, int log2_homes,
+                                                       int do_tick, int nsims, SimParams *sims, double *red) {
+    step_kernel_begin();
     if (do_tick)
         for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nsims; k += gridDim.x * blockDim.x) tick(sims[k], red);
     const int c = blockIdx.x * kScanCells + 4 * threadIdx.x;
@@ -268,7 +269,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(int ncells, int32_t *coun
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         m[k] = c + k < ncells ? count[c + k] : 0;
-        v += (unsigned long long)cell_items(m[k]) << 32 | (unsigned)m[k];
+        v += (unsigned long long)cell_items(m[k], log2_homes) << 32 | (unsigned)m[k];
     }
     unsigned long long tot, ex = block_scan2(v, &tot);
 #pragma unroll
@@ -276,7 +277,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(int ncells, int32_t *coun
         if (c + k < ncells) {
             part[c + k] = ex;
             if (m[k]) count[c + k] = 0;
-            ex += (unsigned long long)cell_items(m[k]) << 32 | (unsigned)m[k];
+            ex += (unsigned long long)cell_items(m[k], log2_homes) << 32 | (unsigned)m[k];
         }
     __shared__ bool last;
     if (threadIdx.x == 0) {
@@ -304,14 +305,15 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(int ncells, int32_t *coun
 
 __global__ void k_place(int n, int ncells, const int32_t *cell, const int32_t *lidx, const unsigned long long *part,
                         const unsigned long long *pre, int nb, const float4 *aux, int32_t *start, int2 *items,
-                        int *nitems, int2 *tmp) {
+                        int *nitems, int2 *tmp, int log2_homes) {
+    step_kernel_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < ncells) {
         const unsigned long long a = part[i] + pre[i / kScanCells];
         const unsigned long long b = i + 1 < ncells ? part[i + 1] + pre[(i + 1) / kScanCells] : pre[nb];
         start[i] = (int)(unsigned)a;
         const int i0 = (int)(a >> 32), i1 = (int)(b >> 32);
-        for (int k = i0; k < i1; k++) items[k] = make_int2(i, 32 * (k - i0));
+        for (int k = i0; k < i1; k++) items[k] = make_int2(i, (k - i0) << log2_homes);
         if (i == ncells - 1) {
             start[ncells] = (int)(unsigned)b;
             *nitems = i1;
@@ -328,9 +330,10 @@ __global__ void k_place(int n, int ncells, const int32_t *cell, const int32_t *l
 // deterministic order inside a cell) gives the slot its state moves to.  kExt: some simulation
 // has external forces; kRand: some type has had a random force (its persistent value moves).
 template <bool kExt, bool kRand>
-__global__ void k_rank_scatter(int n, int cap, int nspec, const int2 *__restrict__ tmp, const int32_t *__restrict__ start,
+__global__ void k_rank_scatter(int n, int cap, int nspec, const int2 *tmp, const int32_t *start,
                                ParticleArrays src, ParticleArrays dst, int32_t *slot_of_id, const SimParams *sims,
                                const int32_t *cell_sim, const float4 *rforce, float4 *force, float4 *oldx) {
+    step_kernel_begin();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     const int2 me = tmp[t];
@@ -385,7 +388,10 @@ __global__ void k_rank_scatter(int n, int cap, int nspec, const int2 *__restrict
 // bond_eval (tfBond.cpp:97-345) for table potentials; one thread per bond.
 __global__ void k_bonds(int nb, const SimParams *sims, const int32_t *cell_sim, const int2 *bonds,
                         const int32_t *bslot, const PotDev *bpots, const float *bblob, const int32_t *slot_of_id,
-                        const float4 *pos, const float4 *aux, const int32_t *cell, float4 *force, double *red) {
+                        const float4 *pos, const float4 *aux, const int32_t *cell, float4 *force, double *red,
+                        unsigned long long *stamp) {
+    step_kernel_begin();
+    stamp_begin(stamp);
     int b = blockIdx.x * blockDim.x + threadIdx.x;
     float epot = 0.f, vir = 0.f;
     int rb = -1;
@@ -436,7 +442,9 @@ __global__ void k_bonds(int nb, const SimParams *sims, const int32_t *cell_sim, 
 // angle_eval (tfAngle.cpp:90-382); one thread per angle, j is the vertex.
 __global__ void k_angles(int na, const SimParams *sims, const int32_t *cell_sim, const int4 *angles,
                          const PotDev *bpots, const float *bblob, const int32_t *slot_of_id, const float4 *pos,
-                         const int32_t *cell, float4 *force, double *red) {
+                         const int32_t *cell, float4 *force, double *red, unsigned long long *stamp) {
+    step_kernel_begin();
+    stamp_begin(stamp);
     int q = blockIdx.x * blockDim.x + threadIdx.x;
     float epot = 0.f;
     int rb = -1;
@@ -528,11 +536,16 @@ __device__ __forceinline__ float advance_verlet(const SimParams &P, bool newtoni
     return __fadd_rn(__fadd_rn(__fmul_rn(w0, w0), __fmul_rn(w1, w1)), __fmul_rn(w2, w2));
 }
 
+constexpr unsigned kStampBlocks = 2048;   // more than two waves of resident blocks
+
 // cell_advance_forward_euler + Fluxes_integrate; one thread per particle.
 __global__ void k_advance(int n, int cap, int nspec, SimParams *sims, const int32_t *cell_sim, float4 *pos,
                           float4 *vel, const float4 *aux, const float4 *force, int32_t *cell, float *sval, float *sq,
                           const float *type_mass, const int32_t *type_dyn, const uint32_t *species_flags,
-                          const float4 *oldx, double *red, uint32_t *err) {
+                          const float4 *oldx, double *red, uint32_t *err, unsigned long long *stamps, int stamp_mask) {
+    step_kernel_begin();
+    for (int k = 2; k < 4; k++)
+        if (stamp_mask & (1 << k)) stamp_begin(stamps + k);
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     float ke = 0.f, vol = 0.f, mig = 0.f;
     float stot[kMaxSpecies];
@@ -680,10 +693,13 @@ reduce:
     }
     keyed_add3(red, rb, RED_KINETIC, ke, RED_VOLUME, vol, RED_MIGRATIONS, mig);
     for (int s = 0; s < nspec; s++) keyed_add(red, rb, RED_SPECIES0 + s, stot[s]);
+    // the end of the step: the latest of the blocks that can end last
+    if (stamp_mask && threadIdx.x == 0 && blockIdx.x + kStampBlocks >= gridDim.x) atomicMax(stamps + 4, global_timer());
 }
 
 __global__ void k_flux_integrate(int n, int cap, int nspec, int sub, const SimParams *sims, const int32_t *cell_sim,
                                  const int32_t *cell, float *sval, float *sq, const uint32_t *species_flags) {
+    step_kernel_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const SimParams &P = sims[cell_sim[cell[i]]];
@@ -752,17 +768,19 @@ int scan_blocks(int ncells) { return nblk(ncells, kScanCells); }
 
 void launch_bin(const BinArgs &b, cudaStream_t s) {
     if (b.n > 0)
-        k_bin_count<<<nblk(b.n, kThreads), kThreads, 0, s>>>(b.n, b.sims, b.cell_sim, b.src.pos, b.src.cell, b.count,
-                                                            b.lidx, b.shuffle);
+        launch_step_kernel(k_bin_count, nblk(b.n, kThreads), kThreads, 0, s, b.n, b.sims, b.cell_sim, b.src.pos,
+                           b.src.cell, b.count, b.lidx, b.shuffle, b.stamp);
     const int nb = scan_blocks(b.ncells);
-    k_scan<<<nb, kScanThreads, 0, s>>>(b.ncells, b.count, b.part, b.pre, b.ticket, b.shuffle, b.nsims, b.sims, b.red);
-    k_place<<<nblk(b.n > b.ncells ? b.n : b.ncells, kThreads), kThreads, 0, s>>>(
-        b.n, b.ncells, b.src.cell, b.lidx, b.part, b.pre, nb, b.src.aux, b.start, b.items, b.nitems, b.tmp);
+    launch_step_kernel(k_scan, nb, kScanThreads, 0, s, b.ncells, b.count, b.part, b.pre, b.ticket, b.log2_homes, b.shuffle,
+                       b.nsims, b.sims, b.red);
+    launch_step_kernel(k_place, nblk(b.n > b.ncells ? b.n : b.ncells, kThreads), kThreads, 0, s, b.n, b.ncells,
+                       b.src.cell, b.lidx, b.part, b.pre, nb, b.src.aux, b.start, b.items, b.nitems, b.tmp,
+                       b.log2_homes);
     if (b.n <= 0) return;
     const int g = nblk(b.n, kThreads);
 #define TFG_SCATTER(E, R)                                                                                       \
-    k_rank_scatter<E, R><<<g, kThreads, 0, s>>>(b.n, b.cap, b.nspec, b.tmp, b.start, b.src, b.dst, b.slot_of_id, \
-                                                b.sims, b.cell_sim, b.rforce, b.force, b.oldx)
+    launch_step_kernel(k_rank_scatter<E, R>, g, kThreads, 0, s, b.n, b.cap, b.nspec, b.tmp, b.start, b.src, b.dst, \
+                       b.slot_of_id, b.sims, b.cell_sim, b.rforce, b.force, b.oldx)
     if (b.has_ext && b.has_rand) TFG_SCATTER(true, true);
     else if (b.has_ext) TFG_SCATTER(true, false);
     else if (b.has_rand) TFG_SCATTER(false, true);
@@ -772,35 +790,37 @@ void launch_bin(const BinArgs &b, cudaStream_t s) {
 
 void launch_bonds(int nb, const SimParams *sims, const int32_t *cell_sim, const int2 *bonds, const int32_t *bslot,
                   const PotDev *bpots, const float *bblob, const int32_t *slot_of_id, const float4 *pos,
-                  const float4 *aux, const int32_t *cell, float4 *force, double *red, cudaStream_t s) {
+                  const float4 *aux, const int32_t *cell, float4 *force, double *red, unsigned long long *stamp,
+                  cudaStream_t s) {
     if (nb > 0)
-        k_bonds<<<nblk(nb, kThreads), kThreads, 0, s>>>(nb, sims, cell_sim, bonds, bslot, bpots, bblob, slot_of_id, pos,
-                                                       aux, cell, force, red);
+        launch_step_kernel(k_bonds, nblk(nb, kThreads), kThreads, 0, s, nb, sims, cell_sim, bonds, bslot, bpots, bblob,
+                           slot_of_id, pos, aux, cell, force, red, stamp);
 }
 
 void launch_angles(int na, const SimParams *sims, const int32_t *cell_sim, const int4 *angles, const PotDev *bpots,
                    const float *bblob, const int32_t *slot_of_id, const float4 *pos, const int32_t *cell,
-                   float4 *force, double *red, cudaStream_t s) {
+                   float4 *force, double *red, unsigned long long *stamp, cudaStream_t s) {
     if (na > 0)
-        k_angles<<<nblk(na, kThreads), kThreads, 0, s>>>(na, sims, cell_sim, angles, bpots, bblob, slot_of_id, pos, cell,
-                                                        force, red);
+        launch_step_kernel(k_angles, nblk(na, kThreads), kThreads, 0, s, na, sims, cell_sim, angles, bpots, bblob,
+                           slot_of_id, pos, cell, force, red, stamp);
 }
 
 void launch_advance(int n, int cap, int nspec, SimParams *sims, const int32_t *cell_sim,
                     const ParticleArrays &A, const float4 *force, const float *type_mass, const int32_t *type_dyn,
-                    const uint32_t *species_flags, const float4 *oldx, double *red, uint32_t *err, cudaStream_t s) {
+                    const uint32_t *species_flags, const float4 *oldx, double *red, uint32_t *err,
+                    unsigned long long *stamps, int stamp_mask, cudaStream_t s) {
     if (n > 0)
-        k_advance<<<nblk(n, kThreads), kThreads, 0, s>>>(n, cap, nspec, sims, cell_sim, A.pos, A.vel, A.aux, force,
-                                                        A.cell, A.sval, A.sq, type_mass, type_dyn, species_flags, oldx,
-                                                        red, err);
+        launch_step_kernel(k_advance, nblk(n, kThreads), kThreads, 0, s, n, cap, nspec, sims, cell_sim, A.pos, A.vel,
+                           A.aux, force, A.cell, A.sval, A.sq, type_mass, type_dyn, species_flags, oldx, red, err,
+                           stamps, stamp_mask);
 }
 
 void launch_flux_integrate(int n, int cap, int nspec, int sub, const SimParams *sims, const int32_t *cell_sim,
                            const int32_t *cell, float *sval, float *sq, const uint32_t *species_flags,
                            cudaStream_t s) {
     if (n > 0 && nspec > 0)
-        k_flux_integrate<<<nblk(n, kThreads), kThreads, 0, s>>>(n, cap, nspec, sub, sims, cell_sim, cell, sval, sq,
-                                                                species_flags);
+        launch_step_kernel(k_flux_integrate, nblk(n, kThreads), kThreads, 0, s, n, cap, nspec, sub, sims, cell_sim,
+                           cell, sval, sq, species_flags);
 }
 
 void launch_gather(int n, int slot0, int cap, int nspec, const SimParams &P, const ParticleArrays &A,

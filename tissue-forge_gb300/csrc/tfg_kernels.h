@@ -23,16 +23,18 @@ struct BinArgs {
     int2 *tmp;                       // (id, slot before) in cell order
     unsigned long long *part, *pre;  // scan scratch: ncells, scan_blocks(ncells) + 1
     unsigned *ticket;
-    int2 *items;                     // the pair pass's work: (cell, first of up to 32 home particles)
+    int2 *items;                     // the pair pass's work: (cell, first of up to 2^log2_homes home particles)
+    int log2_homes;
     int *nitems;
     const float4 *rforce;
     float4 *force;
     float4 *oldx;   // Verlet reference positions by slot (written on rebuild steps), or null
+    unsigned long long *stamp;   // where the binning's begin is stamped, or null
 };
 
 int scan_blocks(int ncells);
-// One thread writes the GPU global timer (ns) into t[k]: phase boundaries of a step, valid
-// inside captured graphs (event timing is not).
+// One thread writes the GPU global timer (ns) into t[k].  The phase boundaries of a step are
+// stamped by its kernels where they can be (null: not at all); this is for the others.
 void launch_stamp(unsigned long long *t, int k, cudaStream_t s);
 void launch_setpartp(int n, const float *xg, const SimParams &P, float3 lo, float3 hi, float3 org, float3 ih,
                      int slot0, int32_t *cell, float4 *pos, float4 *aux, const int32_t *type, uint32_t *err,
@@ -42,13 +44,16 @@ void launch_relocate(int n, int src0, int dst0, int cap_src, int cap_dst, int ns
 void launch_bin(const BinArgs &b, cudaStream_t s);
 void launch_bonds(int nb, const SimParams *sims, const int32_t *cell_sim, const int2 *bonds, const int32_t *bslot,
                   const PotDev *bpots, const float *bblob, const int32_t *slot_of_id, const float4 *pos,
-                  const float4 *aux, const int32_t *cell, float4 *force, double *red, cudaStream_t s);
+                  const float4 *aux, const int32_t *cell, float4 *force, double *red, unsigned long long *stamp,
+                  cudaStream_t s);
 void launch_angles(int na, const SimParams *sims, const int32_t *cell_sim, const int4 *angles, const PotDev *bpots,
                    const float *bblob, const int32_t *slot_of_id, const float4 *pos, const int32_t *cell,
-                   float4 *force, double *red, cudaStream_t s);
+                   float4 *force, double *red, unsigned long long *stamp, cudaStream_t s);
+// stamp_mask: bit k (2, 3) stamps the kernel's begin into stamps[k]; when not 0, its end into stamps[4].
 void launch_advance(int n, int cap, int nspec, SimParams *sims, const int32_t *cell_sim,
                     const ParticleArrays &A, const float4 *force, const float *type_mass, const int32_t *type_dyn,
-                    const uint32_t *species_flags, const float4 *oldx, double *red, uint32_t *err, cudaStream_t s);
+                    const uint32_t *species_flags, const float4 *oldx, double *red, uint32_t *err,
+                    unsigned long long *stamps, int stamp_mask, cudaStream_t s);
 // Fluxes_integrate of flux substep `sub` over every particle of the simulations that have
 // that substep (tf_engine_advance.cpp:314-323, tfFlux.cpp:175-202).
 void launch_flux_integrate(int n, int cap, int nspec, int sub, const SimParams *sims, const int32_t *cell_sim,
