@@ -364,6 +364,7 @@ int upload_tables(tfg_engine *eng) {
     for (auto &f : fl) std::memset(&f, 0, sizeof(f));
     eng->has_dpd = false;
     eng->has_flux = false;
+    eng->radii = false;
     eng->max_fluxsteps = 1;
     uint32_t nodens = TFG_ENGINE_NO_DENSITY;
     for (size_t q = 0; q < eng->order.size(); q++) {
@@ -385,6 +386,7 @@ int upload_tables(tfg_engine *eng) {
                 }
             }
             if (d.kind == POT_DPD) eng->has_dpd = true;
+            if (d.kind == POT_TABLE && (d.flags & (TFG_POTENTIAL_SHIFTED | TFG_POTENTIAL_SCALED))) eng->radii = true;
             if (S.fluxes[k].count > 0) {
                 eng->has_flux = true;
                 eng->max_fluxsteps = std::max(eng->max_fluxsteps, S.P.nr_fluxsteps);
@@ -412,7 +414,7 @@ int upload_tables(tfg_engine *eng) {
         }
     }
     eng->flags_all = nodens;
-    if (blob.empty()) blob.push_back(0.f);
+    if (blob.empty()) blob.assign(kChunk, 0.f);   // row 0 of no table is readable
     int rc;
     if ((rc = ensure(eng, &eng->blob, eng->blob_cap, blob.size())) ||
         (rc = ensure(eng, &eng->pots, eng->pots_cap, pots.size())) ||
@@ -835,6 +837,7 @@ PairKernelArgs pair_args(tfg_engine *eng) {
     a.red = eng->red;
     a.err = eng->err;
     a.has_dpd = eng->has_dpd;
+    a.radii = eng->radii;
     a.flux_sub = -1;
     a.has_flux = eng->has_flux;
     return a;

@@ -111,7 +111,7 @@ struct tfg_engine {
     bool phase_timing = true;
     std::string last_error;
     bool layout_dirty = true, tables_dirty = true;
-    bool has_dpd = false, has_flux = false;
+    bool has_dpd = false, has_flux = false, radii = false;
     int max_fluxsteps = 1;           // largest nr_fluxsteps of a simulation with fluxes
     uint32_t flags_all = 0;          // TFG_ENGINE_NO_DENSITY only when every simulation sets it
     int split = 0;                   // tiled pair pass: warps per home cell (0 = not tuned)

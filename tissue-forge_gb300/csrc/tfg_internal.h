@@ -98,6 +98,7 @@ struct PairKernelArgs {
     int flux_sub;               // >= 0: flux-only substep pass number (simulations with
                                 // nr_fluxsteps - 1 > flux_sub take part); -1: the full pass
     bool has_dpd;               // any type pair uses a DPD potential
+    bool radii;                 // any table is shifted or scaled by the particles' radii
     bool has_flux;              // any type pair has fluxes
 };
 
