@@ -474,16 +474,34 @@ static int err_code(uint32_t flags) {
     return TFG_OK;
 }
 
+// Copy the device error words to the host, in stream order (collect_errors reads them).
+static int fetch_errors(tfg_engine *eng) {
+    const size_t words = 1 + (size_t)std::min((int)eng->order.size(), eng->err_slots);
+    if (words > eng->err_host_cap) {
+        if (eng->err_host) cudaFreeHost(eng->err_host);
+        eng->err_host = nullptr;
+        eng->err_host_cap = 0;
+        CK(cudaMallocHost((void **)&eng->err_host, sizeof(uint32_t) * words));
+        eng->err_host_cap = words;
+    }
+    CK(cudaMemcpyAsync(eng->err_host, eng->err, sizeof(uint32_t) * words, cudaMemcpyDeviceToHost, eng->stream));
+    return TFG_OK;
+}
+
 // Read and clear the device error words.  A simulation's word goes to its sticky status
 // (the reference flags the offending particle, toofast_error, tf_engine_advance.cpp:72-85,
 // 204-206; here the simulation is the unit that fails), the engine's word to pending_err.
-int collect_errors(tfg_engine *eng) {
+// `fetched`: fetch_errors was called and the stream has been waited for since.
+int collect_errors(tfg_engine *eng, bool fetched) {
+    if (!fetched) {
+        int rc = fetch_errors(eng);
+        if (rc) return rc;
+        CK(cudaStreamSynchronize(eng->stream));
+    }
     const int ns = std::min((int)eng->order.size(), eng->err_slots);
-    std::vector<uint32_t> w(1 + ns, 0u);
-    CK(cudaMemcpyAsync(w.data(), eng->err, sizeof(uint32_t) * (1 + ns), cudaMemcpyDeviceToHost, eng->stream));
-    CK(cudaStreamSynchronize(eng->stream));
+    const uint32_t *w = eng->err_host;
     bool any = false;
-    for (uint32_t x : w) any |= x != 0u;
+    for (int k = 0; k <= ns; k++) any |= w[k] != 0u;
     if (!any) return TFG_OK;
     CK(cudaMemsetAsync(eng->err, 0, sizeof(uint32_t) * (1 + ns), eng->stream));
     CK(cudaStreamSynchronize(eng->stream));
@@ -495,8 +513,8 @@ int collect_errors(tfg_engine *eng) {
     return TFG_OK;
 }
 
-int read_err(tfg_engine *eng) {
-    int rc = collect_errors(eng);
+int read_err(tfg_engine *eng, bool fetched) {
+    int rc = collect_errors(eng, fetched);
     if (rc) return rc;
     const uint32_t flags = eng->pending_err;
     eng->pending_err = 0u;
@@ -1099,31 +1117,28 @@ int download_sim(tfg_engine *eng, int sim, float *x, float *xrel, int32_t *cell,
     const int n = S.n, ns = eng->nspec;
     if (n == 0) return TFG_OK;
     cudaStream_t s = eng->stream;
-    const size_t nf = (size_t)n * (3 + 3 + 3 + 3 + 1 + 2 * ns) + n;
-    float *stage = nullptr;
-    if ((rc = dalloc(eng, &stage, nf))) return rc;
-    float *dx = stage, *dxr = dx + 3 * n, *dv = dxr + 3 * n, *df = dv + 3 * n, *dd = df + 3 * n;
-    float *dsp = dd + n, *dq = dsp + (size_t)n * ns;
-    int32_t *dc = reinterpret_cast<int32_t *>(dq + (size_t)n * ns);
-    launch_gather(n, S.P.id_off, eng->cap, ns, S.P, eng->A[eng->cur], eng->force, dx, dxr, dc, dv, df, dd,
-                  ns ? dsp : nullptr, ns ? dq : nullptr, s);
-    auto cp = [&](void *dst, const void *src, size_t bytes) {
-        if (dst) cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s);
-    };
-    cp(x, dx, sizeof(float) * 3 * n);
-    cp(xrel, dxr, sizeof(float) * 3 * n);
-    cp(v, dv, sizeof(float) * 3 * n);
-    cp(f, df, sizeof(float) * 3 * n);
-    cp(dens, dd, sizeof(float) * n);
-    if (ns) {
-        cp(species, dsp, sizeof(float) * n * ns);
-        cp(q, dq, sizeof(float) * n * ns);
-    }
-    cp(cell, dc, sizeof(int32_t) * n);
-    cudaError_t e = cudaStreamSynchronize(s);
-    cudaFree(stage);
-    if (e != cudaSuccess) return fail(eng, TFG_E_CUDA, cudaGetErrorString(e));
-    return read_err(eng);
+    // the wanted arrays are gathered into a buffer that the engine keeps (it grows to the
+    // largest download), then copied
+    struct { float *host, *dev; size_t count; } out[8] = {
+        {x, nullptr, (size_t)3 * n},  {xrel, nullptr, (size_t)3 * n}, {v, nullptr, (size_t)3 * n},
+        {f, nullptr, (size_t)3 * n},  {dens, nullptr, (size_t)n},     {ns ? species : nullptr, nullptr, (size_t)n * ns},
+        {ns ? q : nullptr, nullptr, (size_t)n * ns}, {reinterpret_cast<float *>(cell), nullptr, (size_t)n}};
+    size_t need = 0;
+    for (auto &o : out) need += o.host ? o.count : 0;
+    if ((rc = ensure(eng, &eng->stage, eng->stage_cap, need))) return rc;
+    size_t at = 0;
+    for (auto &o : out)
+        if (o.host) {
+            o.dev = eng->stage + at;
+            at += o.count;
+        }
+    launch_gather(n, S.P.id_off, eng->cap, ns, S.P, eng->A[eng->cur], eng->force, out[0].dev, out[1].dev,
+                  reinterpret_cast<int32_t *>(out[7].dev), out[2].dev, out[3].dev, out[4].dev, out[5].dev, out[6].dev, s);
+    for (const auto &o : out)
+        if (o.host) CK(cudaMemcpyAsync(o.host, o.dev, sizeof(float) * o.count, cudaMemcpyDeviceToHost, s));
+    if ((rc = fetch_errors(eng))) return rc;
+    CK(cudaStreamSynchronize(s));
+    return read_err(eng, true);
 }
 
 int reductions_sim(tfg_engine *eng, int sim, tfg_reductions *out) {
@@ -1136,6 +1151,7 @@ int reductions_sim(tfg_engine *eng, int sim, tfg_reductions *out) {
     if (!S.in_arena) return TFG_OK;
     double r[RED_COUNT];
     CK(cudaMemcpyAsync(r, eng->red + S.P.red_base, sizeof(r), cudaMemcpyDeviceToHost, eng->stream));
+    if ((rc = fetch_errors(eng))) return rc;
     CK(cudaStreamSynchronize(eng->stream));
     out->epot_nonbond = r[RED_EPOT_NONBOND];
     out->epot_bond = r[RED_EPOT_BOND];
@@ -1146,7 +1162,7 @@ int reductions_sim(tfg_engine *eng, int sim, tfg_reductions *out) {
     out->computed_volume = r[RED_VOLUME];
     for (int k = 0; k < kMaxSpecies; k++) out->species_total[k] = r[RED_SPECIES0 + k];
     out->migrations = (int64_t)r[RED_MIGRATIONS];
-    return read_err(eng);
+    return read_err(eng, true);
 }
 
 int verlet_sim(tfg_engine *eng, int sim, int64_t *rebuilds, float *maxdx) {
@@ -1175,10 +1191,11 @@ void destroy(tfg_engine *eng) {
                     eng->slot_of_id, eng->scan_part, eng->scan_pre, eng->counters, eng->cell_sim,
                     eng->sims_dev, eng->corig, eng->pots, eng->potc, eng->blob, eng->fluxes, eng->rforce, eng->type_mass,
                     eng->type_dyn, eng->species_flags, eng->bonds, eng->bond_slot, eng->angles, eng->bpots,
-                    eng->bblob, eng->red, eng->err, eng->oldx};
+                    eng->bblob, eng->red, eng->err, eng->oldx, eng->stage};
     for (void *p : bufs) cudaFree(p);
     for (int k = 0; k < 5; k++)
         if (eng->ev[k]) cudaEventDestroy(eng->ev[k]);
+    if (eng->err_host) cudaFreeHost(eng->err_host);
     if (eng->own_stream && eng->stream) cudaStreamDestroy(eng->stream);
     delete eng;
 }

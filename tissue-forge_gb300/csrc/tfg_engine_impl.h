@@ -103,6 +103,10 @@ struct tfg_engine {
     // slot q (order[q]); collected into SimHost::status and pending_err at every read
     uint32_t *err = nullptr;
     int err_slots = 0;               // simulation words allocated after err[0]
+    uint32_t *err_host = nullptr;    // pinned copy of the error words
+    size_t err_host_cap = 0;
+    float *stage = nullptr;          // device staging of downloads
+    size_t stage_cap = 0;
     uint32_t pending_err = 0;        // engine bits collected but not yet reported
     cudaStream_t stream = nullptr;
     bool own_stream = false;
@@ -149,8 +153,8 @@ template <typename T> int dalloc(tfg_engine *eng, T **p, size_t count) {
     return TFG_OK;
 }
 int check_launch(tfg_engine *eng);
-int read_err(tfg_engine *eng);
-int collect_errors(tfg_engine *eng);            // device error words -> SimHost::status, pending_err
+int read_err(tfg_engine *eng, bool fetched = false);
+int collect_errors(tfg_engine *eng, bool fetched = false);  // device error words -> SimHost::status, pending_err
 int sim_status(tfg_engine *eng, int sim, int *status);
 int sim_check(tfg_engine *eng, int sim);        // TFG_OK when `sim` names a live simulation
 int add_sim(tfg_engine *eng, const tfg_engine_desc *d, int *out);
