@@ -273,9 +273,7 @@ __device__ __forceinline__ float density_w(float r, float inv_h, float norm) {
 // One interval of a table (potential_eval_ex's polynomial, tf_potential_eval.h:128-139):
 // x = (r - c0) c1, ee and eff by the Horner recurrence over c2..c7.  The row is 8 floats,
 // 32-byte aligned (table offsets are multiples of 8), read as two 128-bit loads.
-__device__ __forceinline__ void table_row_eval(const float *row, float r, float &ee, float &eff, float &c1) {
-    const float4 *c4 = reinterpret_cast<const float4 *>(row);
-    const float4 ca = c4[0], cb = c4[1];
+__device__ __forceinline__ void table_row_eval(const float4 &ca, const float4 &cb, float r, float &ee, float &eff) {
     const float x = (r - ca.x) * ca.y;
     ee = fmaf(ca.z, x, ca.w);
     eff = ca.z;
@@ -287,6 +285,11 @@ __device__ __forceinline__ void table_row_eval(const float *row, float r, float 
     ee = fmaf(ee, x, cb.z);
     eff = fmaf(eff, x, ee);
     ee = fmaf(ee, x, cb.w);
+}
+__device__ __forceinline__ void table_row_eval(const float *row, float r, float &ee, float &eff, float &c1) {
+    const float4 *c4 = reinterpret_cast<const float4 *>(row);
+    const float4 ca = c4[0], cb = c4[1];
+    table_row_eval(ca, cb, r, ee, eff);
     c1 = ca.y;
 }
 

@@ -235,13 +235,20 @@ int relayout(tfg_engine *eng) {
     orig_all.reserve(norig);
     std::vector<SimParams> P_all;
     std::vector<int32_t> cell_sim(std::max(C, 1), 0);
+    std::vector<int4> cell_at(std::max(C, 1), make_int4(0, 0, 0, 0));
     for (size_t q = 0; q < order.size(); q++) {
         SimHost &S = eng->sims[order[q]];
         const size_t base = orig_all.size();
         orig_all.insert(orig_all.end(), S.orig.begin(), S.orig.end());
         for (int k = 0; k < 3; k++) S.P.corig[k] = eng->corig + base + (size_t)k * S.maxc;
         P_all.push_back(S.P);
-        for (int c = 0; c < S.P.ncells; c++) cell_sim[S.P.cell_off + c] = (int32_t)q;
+        int c = S.P.cell_off;
+        for (int i = 0; i < S.P.cdim[0]; i++)
+            for (int j = 0; j < S.P.cdim[1]; j++)
+                for (int k = 0; k < S.P.cdim[2]; k++, c++) {
+                    cell_sim[c] = (int32_t)q;
+                    cell_at[c] = make_int4(i, j, k, (int)q);
+                }
     }
     if (norig) CK(cudaMemcpyAsync(eng->corig, orig_all.data(), sizeof(float) * norig, cudaMemcpyHostToDevice, s));
     if ((int)order.size() > eng->sims_cap) {
@@ -254,12 +261,13 @@ int relayout(tfg_engine *eng) {
         const int cc = C + 1;
         if ((rc = dalloc(eng, &eng->count, cc)) || (rc = dalloc(eng, &eng->start, cc + 1)) ||
             (rc = dalloc(eng, &eng->scan_part, cc)) || (rc = dalloc(eng, &eng->scan_pre, scan_blocks(cc) + 1)) ||
-            (rc = dalloc(eng, &eng->cell_sim, cc)))
+            (rc = dalloc(eng, &eng->cell_sim, cc)) || (rc = dalloc(eng, &eng->cell_at, cc)))
             return rc;
         CK(cudaMemsetAsync(eng->count, 0, sizeof(int32_t) * cc, s));
         eng->cells_cap = cc;
     }
     if ((rc = ensure(eng, &eng->items, eng->items_cap, (size_t)C + N / 8 + 1))) return rc;
+    CK(cudaMemcpyAsync(eng->cell_at, cell_at.data(), sizeof(int4) * std::max(C, 1), cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(eng->cell_sim, cell_sim.data(), sizeof(int32_t) * std::max(C, 1), cudaMemcpyHostToDevice, s));
     if ((int)order.size() > eng->err_slots) {
         const int slots = std::max((int)order.size(), 2 * eng->err_slots);
@@ -822,6 +830,7 @@ PairKernelArgs pair_args(tfg_engine *eng) {
     std::memset(&a, 0, sizeof(a));
     a.sims = eng->sims_dev;
     a.cell_sim = eng->cell_sim;
+    a.cell_at = eng->cell_at;
     a.nsims = (int)eng->order.size();
     a.ncells = eng->ncells;
     a.max_type = eng->max_type;
@@ -1188,7 +1197,7 @@ void destroy(tfg_engine *eng) {
     drop_graphs(eng);
     for (int b = 0; b < 2; b++) free_particles(eng->A[b]);
     void *bufs[] = {eng->wpots, eng->stamps, eng->force, eng->count, eng->start, eng->lidx, eng->bin_tmp, eng->items,
-                    eng->slot_of_id, eng->scan_part, eng->scan_pre, eng->counters, eng->cell_sim,
+                    eng->slot_of_id, eng->scan_part, eng->scan_pre, eng->counters, eng->cell_sim, eng->cell_at,
                     eng->sims_dev, eng->corig, eng->pots, eng->potc, eng->blob, eng->fluxes, eng->rforce, eng->type_mass,
                     eng->type_dyn, eng->species_flags, eng->bonds, eng->bond_slot, eng->angles, eng->bpots,
                     eng->bblob, eng->red, eng->err, eng->oldx, eng->stage};

@@ -59,6 +59,7 @@ struct tfg_engine {
     float4 *oldx = nullptr;          // Verlet reference positions by slot
     int oldx_cap = 0;
     int32_t *count = nullptr, *start = nullptr, *lidx = nullptr, *slot_of_id = nullptr, *cell_sim = nullptr;
+    int4 *cell_at = nullptr;         // per global cell: grid location, simulation
     int2 *bin_tmp = nullptr, *items = nullptr;
     unsigned long long *scan_part = nullptr, *scan_pre = nullptr;
     size_t items_cap = 0;

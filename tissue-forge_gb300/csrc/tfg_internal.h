@@ -57,6 +57,7 @@ enum RedSlot : int {
 struct PairKernelArgs {
     const SimParams *sims;      // per-simulation parameters (device)
     const int32_t *cell_sim;    // simulation of each global cell (device)
+    const int4 *cell_at;        // grid location of each global cell; w: its simulation
     int nsims;
     int ncells;                 // global cells over all simulations
     int max_type;               // types per simulation (tables are max_type^2 per simulation)

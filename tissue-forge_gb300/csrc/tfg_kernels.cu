@@ -197,6 +197,7 @@ __global__ void k_bin_count(int n, const SimParams *sims, const int32_t *cell_si
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     int c = cell[i];
+    float4 p = shuffle ? pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
     if (shuffle) {
         const SimParams &P = sims[cell_sim[c]];
         // Verlet mode re-bins only on rebuild steps (engine_verlet_update -> engine_shuffle);
@@ -205,7 +206,6 @@ __global__ void k_bin_count(int n, const SimParams *sims, const int32_t *cell_si
             lidx[i] = atomicAdd(&count[c], 1);
             return;
         }
-        float4 p = pos[i];
         int d0 = (p.x >= P.h[0]) - (p.x < 0.f);
         int d1 = (p.y >= P.h[1]) - (p.y < 0.f);
         int d2 = (p.z >= P.h[2]) - (p.z < 0.f);
@@ -399,15 +399,27 @@ __global__ void k_bonds(int nb, const SimParams *sims, const int32_t *cell_sim, 
         const int2 bd = bonds[b];
         const PotDev &pot = bpots[bslot[b]];
         const int si = slot_of_id[bd.x], sj = slot_of_id[bd.y];
-        const SimParams *Pp = (si >= 0) ? &sims[cell_sim[cell[si]]] : nullptr;
-        if (pot.kind == POT_TABLE && si >= 0 && sj >= 0 && !Pp->stopped) {
-            const SimParams &P = *Pp;
+        const bool there = pot.kind == POT_TABLE && si >= 0 && sj >= 0;
+        float4 pi = make_float4(0.f, 0.f, 0.f, 0.f), pj = pi;
+        int ci = 0, cj = 0;
+        if (there) {
+            pi = pos[si];
+            pj = pos[sj];
+            ci = cell[si];
+            cj = cell[sj];
+        }
+        const SimParams &P = sims[cell_sim[ci]];
+        if (there && !P.stopped) {
             rb = P.red_base;
-            const float4 pi = pos[si], pj = pos[sj];
-            int ai, bi, ci, aj, bj, cj;
-            cell_loc(P, cell[si], ai, bi, ci);
-            cell_loc(P, cell[sj], aj, bj, cj);
-            const int s0 = wrap_shift(ai - aj), s1 = wrap_shift(bi - bj), s2 = wrap_shift(ci - cj);
+            int s0 = 0, s1 = 0, s2 = 0;
+            if (ci != cj) {
+                int ai, bi, ki, aj, bj, kj;
+                cell_loc(P, ci, ai, bi, ki);
+                cell_loc(P, cj, aj, bj, kj);
+                s0 = wrap_shift(ai - aj);
+                s1 = wrap_shift(bi - bj);
+                s2 = wrap_shift(ki - kj);
+            }
             const float pix = __fadd_rn(pi.x, __fmul_rn(P.h[0], (float)s0));
             const float piy = __fadd_rn(pi.y, __fmul_rn(P.h[1], (float)s1));
             const float piz = __fadd_rn(pi.z, __fmul_rn(P.h[2], (float)s2));
@@ -452,15 +464,24 @@ __global__ void k_angles(int na, const SimParams *sims, const int32_t *cell_sim,
         const int4 A = angles[q];
         const PotDev &pot = bpots[A.w];
         const int si = slot_of_id[A.x], sj = slot_of_id[A.y], sk = slot_of_id[A.z];
-        const SimParams *Pp = (sj >= 0) ? &sims[cell_sim[cell[sj]]] : nullptr;
-        if (pot.kind == POT_TABLE && si >= 0 && sj >= 0 && sk >= 0 && !Pp->stopped) {
-            const SimParams &P = *Pp;
+        const bool there = pot.kind == POT_TABLE && si >= 0 && sj >= 0 && sk >= 0;
+        float4 pi = make_float4(0.f, 0.f, 0.f, 0.f), pj = pi, pk = pi;
+        int ci = 0, cj = 0, ck = 0;
+        if (there) {
+            pi = pos[si];
+            pj = pos[sj];
+            pk = pos[sk];
+            ci = cell[si];
+            cj = cell[sj];
+            ck = cell[sk];
+        }
+        const SimParams &P = sims[cell_sim[cj]];
+        if (there && !P.stopped) {
             rb = P.red_base;
-            const float4 pi = pos[si], pj = pos[sj], pk = pos[sk];
             int li[3], lj[3], lk[3];
-            cell_loc(P, cell[si], li[0], li[1], li[2]);
-            cell_loc(P, cell[sj], lj[0], lj[1], lj[2]);
-            cell_loc(P, cell[sk], lk[0], lk[1], lk[2]);
+            cell_loc(P, ci, li[0], li[1], li[2]);
+            cell_loc(P, cj, lj[0], lj[1], lj[2]);
+            cell_loc(P, ck, lk[0], lk[1], lk[2]);
             float xi[3] = {pi.x, pi.y, pi.z}, xj[3] = {pj.x, pj.y, pj.z}, xk[3] = {pk.x, pk.y, pk.z};
             float rji[3], rjk[3];
             for (int k = 0; k < 3; k++) {
@@ -554,13 +575,19 @@ __global__ void k_advance(int n, int cap, int nspec, SimParams *sims, const int3
     int rb = -1;
     int vsim = -1;          // Verlet simulation of this particle
     uint32_t dx2 = 0u;      // its squared displacement (float bits)
-    if (i < n && !sims[cell_sim[cell[i]]].stopped) {
-        const int c0 = cell[i];
+    // every particle's state is loaded at once, before it is known whether its simulation runs
+    int c0 = 0;
+    float4 p = make_float4(0.f, 0.f, 0.f, 0.f), v = p, ax = p, f = p;
+    if (i < n) {
+        c0 = cell[i];
+        p = pos[i];
+        v = vel[i];
+        ax = aux[i];
+        f = force[i];
+    }
+    if (i < n && !sims[cell_sim[c0]].stopped) {
         const SimParams &P = sims[cell_sim[c0]];
         rb = P.red_base;
-        float4 p = pos[i], v = vel[i];
-        const float4 ax = aux[i];
-        const float4 f = force[i];
         const int type = __float_as_int(p.w);
         const uint32_t flags = (uint32_t)__float_as_int(ax.z);
         const float imass = ax.y;
