@@ -49,6 +49,14 @@ struct SimHost {
     std::vector<float> q_pending;    // flux increments to restore at the next layout (id order)
 };
 
+// A captured graph of one step or of kGraphSteps steps.
+struct StepGraph {
+    cudaGraphExec_t exec = nullptr;
+    uint64_t gen = 0;
+    int next = 0;                    // buffer index after a replay
+};
+constexpr int kGraphSteps = 4, kGraphAfter = 16;
+
 struct tfg_engine {
     int device = 0, max_type = 1, nspec = 0, sms = 1;
     std::vector<SimHost> sims;       // by simulation id; removed ones have live == false
@@ -132,9 +140,8 @@ struct tfg_engine {
     // captured again, after one eager step of the new generation (`eager_gen`).
     bool use_graphs = true;
     uint64_t gen = 1;
-    uint64_t graph_gen[2] = {0, 0};
-    cudaGraphExec_t graph[2] = {nullptr, nullptr};
-    int graph_next[2] = {1, 0};      // buffer index after a replay from each parity
+    StepGraph graphs[4];             // [2 * buffer parity + (several steps)]
+    int replayed = 0;                // single steps replayed in this generation
     uint64_t eager_gen = 0;
 };
 
@@ -167,7 +174,7 @@ void advance_clocks(tfg_engine *eng);           // host clocks, by k_tick's rule
 int set_stop_sim(tfg_engine *eng, int sim, int64_t step);
 int enqueue_step(tfg_engine *eng, bool advance, bool timed);
 int flux_substeps(tfg_engine *eng);  // one_step without the host clock
-int graph_step(tfg_engine *eng);                // one step replayed from a captured graph
+int graph_steps(tfg_engine *eng, int steps);    // steps replayed from a captured graph
 int run_steps(tfg_engine *eng, int nsteps);     // nsteps steps, graphs where they apply
 int autotune(tfg_engine *eng, bool splits_only = false);
 int tune_if_needed(tfg_engine *eng);   // first tuning, or a re-tune after the batch grew or shrank 4x
