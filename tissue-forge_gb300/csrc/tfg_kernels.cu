@@ -179,7 +179,7 @@ __global__ void k_relocate(int n, int src0, int dst0, int cap_src, int cap_dst, 
     }
 }
 
-// Binning, in four launches.  It is bound by launches and L2 latency below about 100,000
+// Binning, in four launches (one for small arenas, k_bin_small).  It is bound by launches and L2 latency below about 100,000
 // particles and by HBM above:
 //   k_bin_count    re-check of the cell-relative positions, count per cell
 //   k_scan         block-local scan of the counts; the last block to finish scans the block
@@ -187,41 +187,41 @@ __global__ void k_relocate(int n, int src0, int dst0, int cap_src, int cap_dst, 
 //   k_place        final cell starts, the pair pass's work items, (id, slot) into cell order
 //   k_rank_scatter rank by id inside the cell, then the state itself, with the force init
 
-// Re-check of the cell-relative position (space_shuffle_local) and per-cell counting.  The
-// simulations' clocks advance in the next kernel, so their decisions for this step are
-// taken from the state before it.
+// Re-check of the cell-relative position (space_shuffle_local, tfSpace.cpp:274-391); returns the
+// particle's cell.  The simulations' clocks advance in a later part of the binning, so their
+// decisions for this step are taken from the state before it.
+__device__ __forceinline__ int recheck(int i, const SimParams *sims, const int32_t *cell_sim, float4 *pos,
+                                       int32_t *cell, int shuffle) {
+    int c = cell[i];
+    if (!shuffle) return c;
+    float4 p = pos[i];
+    const SimParams &P = sims[cell_sim[c]];
+    // Verlet mode re-bins only on rebuild steps (engine_verlet_update -> engine_shuffle);
+    // a stopped simulation stays as it is
+    if (stops_now(P) || ((P.flags & TFG_ENGINE_VERLET) && !rebuilds_now(P))) return c;
+    const int d0 = (p.x >= P.h[0]) - (p.x < 0.f);
+    const int d1 = (p.y >= P.h[1]) - (p.y < 0.f);
+    const int d2 = (p.z >= P.h[2]) - (p.z < 0.f);
+    if (d0 | d1 | d2) {
+        p.x = __fsub_rn(p.x, __fmul_rn((float)d0, P.h[0]));
+        p.y = __fsub_rn(p.y, __fmul_rn((float)d1, P.h[1]));
+        p.z = __fsub_rn(p.z, __fmul_rn((float)d2, P.h[2]));
+        pos[i] = p;
+        int a, b, k;
+        cell_loc(P, c, a, b, k);
+        c = cell_index(P, (a + d0 + P.cdim[0]) % P.cdim[0], (b + d1 + P.cdim[1]) % P.cdim[1],
+                       (k + d2 + P.cdim[2]) % P.cdim[2]);
+        cell[i] = c;
+    }
+    return c;
+}
+
 __global__ void k_bin_count(int n, const SimParams *sims, const int32_t *cell_sim, float4 *pos, int32_t *cell,
                             int32_t *count, int32_t *lidx, int shuffle, unsigned long long *stamp) {
     step_kernel_begin();
     stamp_begin(stamp);
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int c = cell[i];
-    float4 p = shuffle ? pos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    if (shuffle) {
-        const SimParams &P = sims[cell_sim[c]];
-        // Verlet mode re-bins only on rebuild steps (engine_verlet_update -> engine_shuffle);
-        // a stopped simulation stays as it is
-        if (stops_now(P) || ((P.flags & TFG_ENGINE_VERLET) && !rebuilds_now(P))) {
-            lidx[i] = atomicAdd(&count[c], 1);
-            return;
-        }
-        int d0 = (p.x >= P.h[0]) - (p.x < 0.f);
-        int d1 = (p.y >= P.h[1]) - (p.y < 0.f);
-        int d2 = (p.z >= P.h[2]) - (p.z < 0.f);
-        if (d0 | d1 | d2) {
-            p.x = __fsub_rn(p.x, __fmul_rn((float)d0, P.h[0]));
-            p.y = __fsub_rn(p.y, __fmul_rn((float)d1, P.h[1]));
-            p.z = __fsub_rn(p.z, __fmul_rn((float)d2, P.h[2]));
-            pos[i] = p;
-            int a, b, k;
-            cell_loc(P, c, a, b, k);
-            c = cell_index(P, (a + d0 + P.cdim[0]) % P.cdim[0], (b + d1 + P.cdim[1]) % P.cdim[1],
-                           (k + d2 + P.cdim[2]) % P.cdim[2]);
-            cell[i] = c;
-        }
-    }
-    lidx[i] = atomicAdd(&count[c], 1);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) lidx[i] = atomicAdd(&count[recheck(i, sims, cell_sim, pos, cell, shuffle)], 1);
 }
 
 constexpr int kScanThreads = 1024, kScanCells = 4 * kScanThreads;   // cells per block
@@ -326,23 +326,18 @@ __global__ void k_place(int n, int ncells, const int32_t *cell, const int32_t *l
     }
 }
 
-// One thread per place p of the cell order: its particle's rank by id among the cell's (the
+// Place t of the cell order holds particle (id, i): its rank by id among the cell's (the
 // deterministic order inside a cell) gives the slot its state moves to.  kExt: some simulation
 // has external forces; kRand: some type has had a random force (its persistent value moves).
 template <bool kExt, bool kRand>
-__global__ void k_rank_scatter(int n, int cap, int nspec, const int2 *tmp, const int32_t *start,
-                               ParticleArrays src, ParticleArrays dst, int32_t *slot_of_id, const SimParams *sims,
-                               const int32_t *cell_sim, const float4 *rforce, float4 *force, float4 *oldx) {
-    step_kernel_begin();
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    const int2 me = tmp[t];
-    const int id = me.x, i = me.y;
-    const int c = src.cell[i];
+__device__ __forceinline__ void rank_and_move(int id, int i, int c, int s0, int s1, int cap, int nspec, const int2 *tmp,
+                                              const ParticleArrays &src, const ParticleArrays &dst,
+                                              int32_t *slot_of_id, const SimParams *sims, const int32_t *cell_sim,
+                                              const float4 *rforce, float4 *force, float4 *oldx) {
     const float4 ax = src.aux[i], p = src.pos[i], v = src.vel[i];
-    const int s0 = start[c], s1 = start[c + 1];
     const SimParams &P = sims[cell_sim[c]];
     int d = s0;
+#pragma unroll 8
     for (int o = s0; o < s1; o++) d += tmp[o].x < id;
     float4 fe = make_float4(0.f, 0.f, 0.f, 0.f);
     if (kExt) {
@@ -383,6 +378,99 @@ __global__ void k_rank_scatter(int n, int cap, int nspec, const int2 *tmp, const
         dst.sq[s * cap + d] = src.sq[s * cap + i];
     }
     if (slot_of_id) slot_of_id[id] = d;
+}
+
+template <bool kExt, bool kRand>
+__global__ void k_rank_scatter(int n, int cap, int nspec, const int2 *tmp, const int32_t *start, ParticleArrays src,
+                               ParticleArrays dst, int32_t *slot_of_id, const SimParams *sims, const int32_t *cell_sim,
+                               const float4 *rforce, float4 *force, float4 *oldx) {
+    step_kernel_begin();
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const int2 me = tmp[t];
+    const int c = src.cell[me.y];
+    rank_and_move<kExt, kRand>(me.x, me.y, c, start[c], start[c + 1], cap, nspec, tmp, src, dst, slot_of_id, sims,
+                               cell_sim, rforce, force, oldx);
+}
+
+// The whole binning of a small arena in one launch, by one cluster of eight blocks.  Four
+// launches take 10 us however few particles there are; this takes two cluster barriers.  Every
+// block scans all counts itself, so the cell starts are in its shared memory.
+constexpr int kSmallBlocks = 8, kSmallThreads = 1024, kSmallPer = 2;   // up to 16,384 particles
+constexpr int kSmallCells = 16 * kSmallThreads;
+
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+template <bool kExt, bool kRand>
+__global__ void __cluster_dims__(kSmallBlocks, 1, 1) __launch_bounds__(kSmallThreads, 1) k_bin_small(BinArgs b) {
+    extern __shared__ int32_t start_s[];
+    step_kernel_begin();
+    stamp_begin(b.stamp);
+    const int t0 = blockIdx.x * kSmallThreads + threadIdx.x;
+    // count
+    int c[kSmallPer], l[kSmallPer], id[kSmallPer];
+#pragma unroll
+    for (int r = 0; r < kSmallPer; r++) {
+        const int i = t0 + r * kSmallBlocks * kSmallThreads;
+        if (i < b.n) {
+            id[r] = __float_as_int(b.src.aux[i].w);
+            c[r] = recheck(i, b.sims, b.cell_sim, b.src.pos, b.src.cell, b.shuffle);
+            l[r] = atomicAdd(&b.count[c[r]], 1);
+        }
+    }
+    cluster_barrier();
+    // scan: thread t holds cells [per t, per (t + 1)); the blocks share the writing
+    const int per = (b.ncells + kSmallThreads - 1) / kSmallThreads, first = per * threadIdx.x;
+    unsigned long long sum = 0;
+    for (int k = 0; k < per; k++)
+        if (first + k < b.ncells) {
+            const int m = __ldcg(&b.count[first + k]);
+            start_s[first + k] = m;
+            sum += (unsigned long long)cell_items(m, b.log2_homes) << 32 | (unsigned)m;
+        }
+    unsigned long long all, run = block_scan2(sum, &all);
+    const bool mine = (threadIdx.x & (kSmallBlocks - 1)) == blockIdx.x;
+    for (int k = 0; k < per; k++)
+        if (first + k < b.ncells) {
+            const int m = start_s[first + k], items = cell_items(m, b.log2_homes);
+            start_s[first + k] = (int)(unsigned)run;
+            if (mine) {
+                b.start[first + k] = (int)(unsigned)run;
+                for (int q = 0; q < items; q++) b.items[(run >> 32) + q] = make_int2(first + k, q << b.log2_homes);
+            }
+            run += (unsigned long long)items << 32 | (unsigned)m;
+        }
+    if (t0 == 0) {
+        b.start[b.ncells] = (int)(unsigned)all;
+        *b.nitems = (int)(all >> 32);
+    }
+    if (b.shuffle)
+        for (int k = t0; k < b.nsims; k += kSmallBlocks * kSmallThreads) tick(b.sims[k], b.red);
+    __syncthreads();
+    // place
+#pragma unroll
+    for (int r = 0; r < kSmallPer; r++) {
+        const int i = t0 + r * kSmallBlocks * kSmallThreads;
+        if (i < b.n) b.tmp[start_s[c[r]] + l[r]] = make_int2(id[r], i);
+    }
+    cluster_barrier();
+    // the counts return to zero; rank and move
+    if (mine)
+        for (int k = 0; k < per; k++)
+            if (first + k < b.ncells) b.count[first + k] = 0;
+#pragma unroll
+    for (int r = 0; r < kSmallPer; r++) {
+        const int t = t0 + r * kSmallBlocks * kSmallThreads;
+        if (t < b.n) {
+            const int2 me = b.tmp[t];
+            const int cc = b.src.cell[me.y];
+            rank_and_move<kExt, kRand>(me.x, me.y, cc, start_s[cc], cc + 1 < b.ncells ? start_s[cc + 1] : b.n, b.cap,
+                                       b.nspec, b.tmp, b.src, b.dst, b.slot_of_id, b.sims, b.cell_sim, b.rforce, b.force,
+                                       b.oldx);
+        }
+    }
 }
 
 // bond_eval (tfBond.cpp:97-345) for table potentials; one thread per bond.
@@ -793,7 +881,14 @@ void launch_relocate(int n, int src0, int dst0, int cap_src, int cap_dst, int ns
 
 int scan_blocks(int ncells) { return nblk(ncells, kScanCells); }
 
-void launch_bin(const BinArgs &b, cudaStream_t s) {
+template <bool kExt, bool kRand> void launch_bin_variant(const BinArgs &b, cudaStream_t s) {
+    if (b.n <= kSmallPer * kSmallBlocks * kSmallThreads && b.ncells <= kSmallCells) {
+        static const cudaError_t attr = cudaFuncSetAttribute(
+            k_bin_small<kExt, kRand>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallCells * (int)sizeof(int32_t));
+        (void)attr;   // a failure shows at the launch
+        launch_step_kernel(k_bin_small<kExt, kRand>, kSmallBlocks, kSmallThreads, sizeof(int32_t) * b.ncells, s, b);
+        return;
+    }
     if (b.n > 0)
         launch_step_kernel(k_bin_count, nblk(b.n, kThreads), kThreads, 0, s, b.n, b.sims, b.cell_sim, b.src.pos,
                            b.src.cell, b.count, b.lidx, b.shuffle, b.stamp);
@@ -803,16 +898,16 @@ void launch_bin(const BinArgs &b, cudaStream_t s) {
     launch_step_kernel(k_place, nblk(b.n > b.ncells ? b.n : b.ncells, kThreads), kThreads, 0, s, b.n, b.ncells,
                        b.src.cell, b.lidx, b.part, b.pre, nb, b.src.aux, b.start, b.items, b.nitems, b.tmp,
                        b.log2_homes);
-    if (b.n <= 0) return;
-    const int g = nblk(b.n, kThreads);
-#define TFG_SCATTER(E, R)                                                                                       \
-    launch_step_kernel(k_rank_scatter<E, R>, g, kThreads, 0, s, b.n, b.cap, b.nspec, b.tmp, b.start, b.src, b.dst, \
-                       b.slot_of_id, b.sims, b.cell_sim, b.rforce, b.force, b.oldx)
-    if (b.has_ext && b.has_rand) TFG_SCATTER(true, true);
-    else if (b.has_ext) TFG_SCATTER(true, false);
-    else if (b.has_rand) TFG_SCATTER(false, true);
-    else TFG_SCATTER(false, false);
-#undef TFG_SCATTER
+    if (b.n > 0)
+        launch_step_kernel(k_rank_scatter<kExt, kRand>, nblk(b.n, kThreads), kThreads, 0, s, b.n, b.cap, b.nspec, b.tmp,
+                           b.start, b.src, b.dst, b.slot_of_id, b.sims, b.cell_sim, b.rforce, b.force, b.oldx);
+}
+
+void launch_bin(const BinArgs &b, cudaStream_t s) {
+    if (b.has_ext && b.has_rand) launch_bin_variant<true, true>(b, s);
+    else if (b.has_ext) launch_bin_variant<true, false>(b, s);
+    else if (b.has_rand) launch_bin_variant<false, true>(b, s);
+    else launch_bin_variant<false, false>(b, s);
 }
 
 void launch_bonds(int nb, const SimParams *sims, const int32_t *cell_sim, const int2 *bonds, const int32_t *bslot,
