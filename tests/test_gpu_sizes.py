@@ -1,6 +1,6 @@
 """The binning and the tiled pair pass at the sizes where their launches change: arenas of one
-cluster launch or four (16,384 particles and 16,384 cells), 8, 16 or 32 home particles per
-work item (24,000 and 100,000 particles), partly filled groups, windows and tiles, cells of
+cluster launch or four (8,192 particles and 16,384 cells), 8, 16 or 32 home particles per
+work item (24,000 and 140,000, with DPD 250,000 particles), partly filled groups, windows and tiles, cells of
 several items; and the graphs of several steps.  Cells and pair sets bit-exact against the
 oracle, forces and densities at its bar."""
 import dataclasses
@@ -43,10 +43,22 @@ def _sparse(cells):
 
 
 CASES = {"cells_%d" % n: (lambda n=n: _cells(n)) for n in
-         (1, 2, 31, 33, 97, 1000, 8191, 8193, 16384, 16385, 23999, 24000, 99_999, 100_001)}
-CASES.update({"dpd_%d" % n: (lambda n=n: _dpd(n)) for n in (1, 64, 129, 3001, 16385, 24001)})
+         (1, 2, 31, 33, 97, 1000, 8192, 8193, 16385, 23999, 24000, 139_999, 140_001)}
+CASES.update({"dpd_%d" % n: (lambda n=n: _dpd(n)) for n in (1, 64, 129, 3001, 8192, 16385, 24001, 250_001)})
 CASES.update({"clumps_%d" % n: (lambda n=n: _clumps(n)) for n in (150, 1203, 6000, 26_001)})
+# runs of one to four cells along z per work item: few particles a cell, columns of 3 to 9 cells
+CASES.update({"thin_%d" % k: (lambda k=k: _thin(k)) for k in (3, 4, 5, 6, 7, 9)})
 CASES.update({"grid_%dx%dx%d" % c: (lambda c=c: _sparse(c)) for c in ((3, 3, 1820), (3, 3, 1821))})
+
+
+def _thin(k):
+    """1,000 particles, one or two per cell, in a box of k cells along z."""
+    w = configs.lj_fluid(n=1000, seed=k)
+    dim = (2.5 * 18, 2.5 * 1300 // (18 * k) * 1.0 + 10.0, 2.5 * k)
+    rng = np.random.default_rng(k)
+    x = rng.uniform(0.0, 1.0, size=(w.n, 3)) * np.array(dim)
+    cells = tuple(max(3, int(d // 2.5)) for d in dim)
+    return dataclasses.replace(w, x=np.minimum(x, np.array(dim) * (1 - 1e-6)).astype(np.float32), dim=dim, cells=cells)
 
 
 @pytest.mark.parametrize("name", list(CASES))

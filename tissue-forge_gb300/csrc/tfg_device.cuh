@@ -82,8 +82,8 @@ struct SimParams {
     float cutoff, cutoff2;
     // Bound of the tiled pair pass's distance filter x_i - (x_k + shift) above cutoff2.  Each
     // component of it and of the reference's (x_i - shift) - x_k is rounded at a magnitude of
-    // at most twice the cell edge h, so the squares at the cutoff differ by less than
-    // 1.3e-6 h/cutoff + 5e-7 relative; the bound keeps four times that.
+    // at most five cell edges h (a work item spans four cells along z), so the squares at the
+    // cutoff differ by less than 3e-6 h/cutoff + 5e-7 relative; the bound keeps four times that.
     float cut_hi;
     float dt, dt_flux;
     float maxx[3], maxx2[3], maxv[3], maxv2[3], h2[3];

@@ -234,21 +234,12 @@ int relayout(tfg_engine *eng) {
     std::vector<float> orig_all;
     orig_all.reserve(norig);
     std::vector<SimParams> P_all;
-    std::vector<int32_t> cell_sim(std::max(C, 1), 0);
-    std::vector<int4> cell_at(std::max(C, 1), make_int4(0, 0, 0, 0));
     for (size_t q = 0; q < order.size(); q++) {
         SimHost &S = eng->sims[order[q]];
         const size_t base = orig_all.size();
         orig_all.insert(orig_all.end(), S.orig.begin(), S.orig.end());
         for (int k = 0; k < 3; k++) S.P.corig[k] = eng->corig + base + (size_t)k * S.maxc;
         P_all.push_back(S.P);
-        int c = S.P.cell_off;
-        for (int i = 0; i < S.P.cdim[0]; i++)
-            for (int j = 0; j < S.P.cdim[1]; j++)
-                for (int k = 0; k < S.P.cdim[2]; k++, c++) {
-                    cell_sim[c] = (int32_t)q;
-                    cell_at[c] = make_int4(i, j, k, (int)q);
-                }
     }
     if (norig) CK(cudaMemcpyAsync(eng->corig, orig_all.data(), sizeof(float) * norig, cudaMemcpyHostToDevice, s));
     if ((int)order.size() > eng->sims_cap) {
@@ -258,8 +249,9 @@ int relayout(tfg_engine *eng) {
     if (!P_all.empty())
         CK(cudaMemcpyAsync(eng->sims_dev, P_all.data(), sizeof(SimParams) * P_all.size(), cudaMemcpyHostToDevice, s));
     if (C + 1 > eng->cells_cap) {
-        const int cc = C + 1;
-        if ((rc = dalloc(eng, &eng->count, cc)) || (rc = dalloc(eng, &eng->start, cc + 1)) ||
+        const int cc = (C + 4) & ~3;   // the binning takes cells four at a time
+        if ((rc = dalloc(eng, &eng->count, cc)) || (rc = dalloc(eng, &eng->start, cc + 4)) ||
+            (rc = dalloc(eng, &eng->column, cc)) ||
             (rc = dalloc(eng, &eng->scan_part, cc)) || (rc = dalloc(eng, &eng->scan_pre, scan_blocks(cc) + 1)) ||
             (rc = dalloc(eng, &eng->cell_sim, cc)) || (rc = dalloc(eng, &eng->cell_at, cc)))
             return rc;
@@ -267,8 +259,7 @@ int relayout(tfg_engine *eng) {
         eng->cells_cap = cc;
     }
     if ((rc = ensure(eng, &eng->items, eng->items_cap, (size_t)C + N / 8 + 1))) return rc;
-    CK(cudaMemcpyAsync(eng->cell_at, cell_at.data(), sizeof(int4) * std::max(C, 1), cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(eng->cell_sim, cell_sim.data(), sizeof(int32_t) * std::max(C, 1), cudaMemcpyHostToDevice, s));
+    launch_fill_cells((int)order.size(), eng->sims_dev, eng->cell_sim, eng->cell_at, eng->column, s);
     if ((int)order.size() > eng->err_slots) {
         const int slots = std::max((int)order.size(), 2 * eng->err_slots);
         if ((rc = dalloc(eng, &eng->err, 1 + (size_t)slots))) return rc;
@@ -668,7 +659,7 @@ int add_sim(tfg_engine *eng, const tfg_engine_desc *d, int *out) {
     P.ncells = P.cdim[0] * P.cdim[1] * P.cdim[2];
     P.cutoff = d->cutoff;
     P.cutoff2 = d->cutoff * d->cutoff;
-    P.cut_hi = P.cutoff2 * (1.f + 2e-6f + 5e-6f * (std::max(P.h[0], std::max(P.h[1], P.h[2])) / P.cutoff));
+    P.cut_hi = P.cutoff2 * (1.f + 2e-6f + 1.2e-5f * (std::max(P.h[0], std::max(P.h[1], P.h[2])) / P.cutoff));
     P.dt = d->dt;
     const float frac = d->particle_max_dist_fraction > 0 ? d->particle_max_dist_fraction : 0.05f;
     for (int k = 0; k < 3; k++) {
@@ -767,12 +758,21 @@ int load_sim(tfg_engine *eng, int sim, int n, const float *xg, const int32_t *ce
     return TFG_OK;
 }
 
-// Home particles per work item of the tiled pass.  A small arena leaves most warps without an
-// item, and its time is that of the longest one, a crowded cell's: 8 instead of 32 took the
-// pass from 34 to 17 us on 4,000 clustered cells and from 39 to 24 us on 20,000.  More items
-// test more candidates for the same pairs: on 150,001 uniform cells 8, 16 and 32 take 93, 84
-// and 82 us, on 50,000 clustered ones 38, 39 and 46.
-static int log2_homes(const tfg_engine *eng) { return eng->n < 24000 ? 3 : (eng->n < 100000 ? 4 : 5); }
+// Work items of the tiled pass: the most home particles of one, and whether one may span several
+// cells.  A small arena leaves warps without an item, and its time is that of the longest one,
+// a crowded cell's: with 8, 16 and 32 home particles the pass takes 12, 14 and 20 us on 2,000
+// clustered cells, 20, 22 and 32 on 20,000.  Larger items share more: 163, 133 and 120 us on
+// 300,000 uniform cells.  DPD pairs cost more each, so balance counts for longer: 58, 56 and
+// 62 us on 100,000 particles, 136 and 128 (16, 32) on 300,000.
+// Runs of cells share set-up and targets, most where cells hold few particles (DPD droplets
+// that have spread out: 77 -> 38 us), but leave fewer items: on 150,001 uniform cells 67 us
+// without them and 73 with, on
+// 300,000 118 and 121; on LJ fluids of 512,000 and 1,000,000 particles 183 and 180, 351 and 337.
+static void plan_items(tfg_engine *eng) {
+    const bool pairs_cost = eng->has_dpd || (eng->has_flux && eng->nspec > 0);
+    eng->homes = eng->n < 24000 ? 8 : (eng->n < (pairs_cost ? 250000 : 100000) ? 16 : 32);
+    eng->runs = pairs_cost || eng->n >= 450000;
+}
 
 int bin(tfg_engine *eng, int shuffle, bool timed) {
     BinArgs b;
@@ -795,7 +795,10 @@ int bin(tfg_engine *eng, int shuffle, bool timed) {
     b.pre = eng->scan_pre;
     b.ticket = eng->counters;
     b.items = eng->items;
-    b.log2_homes = log2_homes(eng);
+    plan_items(eng);
+    b.column = reinterpret_cast<const uchar4 *>(eng->column);
+    b.homes = eng->homes;
+    b.runs = eng->runs;
     b.nitems = reinterpret_cast<int *>(eng->counters + 1);
     b.nsims = (int)eng->order.size();
     b.red = eng->red;
@@ -845,7 +848,8 @@ PairKernelArgs pair_args(tfg_engine *eng) {
     a.cell = A.cell;
     a.start = eng->start;
     a.items = eng->items;
-    a.homes = 1 << log2_homes(eng);
+    a.homes = eng->homes;   // as the items were listed
+    a.runs = eng->runs;
     a.nitems = reinterpret_cast<const int *>(eng->counters + 1);
     a.counter = eng->counters + 2;
     a.sval = A.sval;
@@ -1049,21 +1053,13 @@ int autotune(tfg_engine *eng, bool splits_only) {
     int rc = dalloc(eng, &save, nq);
     if (rc) return rc;
     CK(cudaMemcpyAsync(save, eng->A[eng->cur].sq, sizeof(float) * nq, cudaMemcpyDeviceToDevice, s));
-    // candidates: every work split of the tiled kernel, in CTAs of 8 warps and, for the table
-    // variants, of 4 (the kernel sizes its grabs itself, so these stay at one item at least)
-    const PairKernelArgs a0 = pair_args(eng);
-    const bool table_only = !a0.has_dpd && !(a0.nspec > 0 && a0.has_flux);
+    // candidates: every work split of the tiled kernel (it sizes its grabs itself)
     std::vector<TileTune> cand;
-    for (int split : {1, 2, 7, 14})
-        for (int warps : {8, 4}) {
-            if (warps == 4 && !table_only) continue;
-            // a re-tune keeps the CTA shape and times the splits only
-            if (splits_only && warps != eng->tune_warps) continue;
-            TileTune t;
-            t.split = split;
-            t.warps = warps;
-            cand.push_back(t);
-        }
+    for (int split : {1, 2, 7, 14}) {
+        TileTune t;
+        t.split = split;
+        cand.push_back(t);
+    }
     // one timed launch of a candidate on freshly initialised forces (ms, or < 0 on error)
     auto trial = [&](const TileTune &tc) -> float {
         rc = bin(eng, 0);
@@ -1206,7 +1202,7 @@ void destroy(tfg_engine *eng) {
     drop_graphs(eng);
     for (int b = 0; b < 2; b++) free_particles(eng->A[b]);
     void *bufs[] = {eng->wpots, eng->stamps, eng->force, eng->count, eng->start, eng->lidx, eng->bin_tmp, eng->items,
-                    eng->slot_of_id, eng->scan_part, eng->scan_pre, eng->counters, eng->cell_sim, eng->cell_at,
+                    eng->slot_of_id, eng->scan_part, eng->scan_pre, eng->counters, eng->cell_sim, eng->cell_at, eng->column,
                     eng->sims_dev, eng->corig, eng->pots, eng->potc, eng->blob, eng->fluxes, eng->rforce, eng->type_mass,
                     eng->type_dyn, eng->species_flags, eng->bonds, eng->bond_slot, eng->angles, eng->bpots,
                     eng->bblob, eng->red, eng->err, eng->oldx, eng->stage};

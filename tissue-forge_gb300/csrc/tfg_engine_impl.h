@@ -68,9 +68,12 @@ struct tfg_engine {
     int oldx_cap = 0;
     int32_t *count = nullptr, *start = nullptr, *lidx = nullptr, *slot_of_id = nullptr, *cell_sim = nullptr;
     int4 *cell_at = nullptr;         // per global cell: grid location, simulation
+    unsigned char *column = nullptr; // per global cell: first of a column along z
     int2 *bin_tmp = nullptr, *items = nullptr;
     unsigned long long *scan_part = nullptr, *scan_pre = nullptr;
     size_t items_cap = 0;
+    int homes = 32;                  // most home particles of a listed work item
+    bool runs = false;               // whether listed items span several cells
     // device counters: [0] scan ticket, [1] work items of the tiled pair pass, [2] its work
     // counter, [3] its finished blocks (each returns to zero by itself, but [1])
     unsigned *counters = nullptr;

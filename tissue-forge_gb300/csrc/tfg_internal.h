@@ -71,9 +71,11 @@ struct PairKernelArgs {
     const float4 *pforce;
     const int32_t *cell;
     const int32_t *start;       // ncells+1
-    const int2 *items;          // work items of the tiled pass: (cell, first of up to `homes` home particles)
+    const int2 *items;          // work items of the tiled pass: (first cell of a run of up to four along z, first of up
+                                // to `homes` home particles | cells - 1 << 30)
     const int *nitems;
     int homes;                  // 8, 16 or 32
+    bool runs;                  // items may span several cells
     unsigned long long *stamp;  // where the pass's begin is stamped, or null
     unsigned *counter;          // work counter of the tiled pass and its finished blocks
     const float *sval;
@@ -108,8 +110,8 @@ struct PairKernelArgs {
 void launch_pair(const PairKernelArgs &a, cudaStream_t s);
 // Launch configuration of the nonbonded pass, picked by the autotuner: the work split (warps
 // per home cell: 1, 2, 7 or 14; the cell's 14 tasks are divided into that many work items;
-// TFG_PAIR_HOME_OUTER means 1), the warps per CTA of the table variants (8, or 4 with twice
-// the CTAs per SM), and the fewest work items a warp takes from the shared counter at a time.
+// TFG_PAIR_HOME_OUTER means 1), the warps per CTA (kept for callers; every CTA has 8), and the
+// fewest work items a warp takes from the shared counter at a time.
 struct TileTune {
     int split = 1;
     int warps = 8;

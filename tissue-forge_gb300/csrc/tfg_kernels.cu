@@ -129,6 +129,18 @@ __device__ __forceinline__ void tick(SimParams &P, double *red) {
     }
 }
 
+// Simulation and grid location of every cell of simulation blockIdx.x.
+__global__ void k_fill_cells(const SimParams *sims, int32_t *cell_sim, int4 *cell_at, unsigned char *column) {
+    const SimParams &P = sims[blockIdx.x];
+    for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < P.ncells; c += gridDim.y * blockDim.x) {
+        int i, j, k;
+        cell_loc(P, P.cell_off + c, i, j, k);
+        cell_sim[P.cell_off + c] = blockIdx.x;
+        cell_at[P.cell_off + c] = make_int4(i, j, k, (int)blockIdx.x);
+        column[P.cell_off + c] = k == 0;
+    }
+}
+
 // space_setpartp (tfSpace.cpp:432-475) for one simulation's particles, written to arena
 // slots [slot0, slot0+n) with global cell indices and ids.
 __global__ void k_setpartp(int n, const float *__restrict__ xg, SimParams P, float3 lo, float3 hi, float3 org,
@@ -252,32 +264,69 @@ __device__ __forceinline__ unsigned long long block_scan2(unsigned long long v, 
     return excl;
 }
 
-// Work items of a cell with n particles: one per 2^log2_homes home particles.
-__device__ __forceinline__ int cell_items(int n, int log2_homes) { return (n + (1 << log2_homes) - 1) >> log2_homes; }
+// Work items of the tiled pair pass from four consecutive cells with m[] particles: runs of
+// neighbouring cells along z (column[k]: cell k is the first of a column) while they hold at most `homes` particles together, or single cells (runs false); a crowded cell is
+// several items.  emit(cell, cells, first home particle, item) is called for each; returns their
+// number.
+template <class F>
+__device__ __forceinline__ int cell_items(const int *m, uchar4 column, int homes, bool runs, F emit) {
+    if (!runs) {
+        int count = 0;
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            for (int c0 = 0; c0 < m[k]; c0 += homes, count++) emit(k, 1, c0, count);
+        return count;
+    }
+    const unsigned char col[4] = {column.x, column.y, column.z, column.w};
+    int first = -1, last = 0, total = 0, count = 0;
+    auto close = [&] {
+        if (first >= 0)
+            for (int c0 = 0; c0 < total; c0 += homes, count++) emit(first, last - first + 1, c0, count);
+        first = -1;
+        total = 0;
+    };
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        if (col[k]) close();
+        if (m[k] == 0) continue;
+        if (total + m[k] > homes) close();
+        if (first < 0) first = k;
+        last = k;
+        total += m[k];
+    }
+    close();
+    return count;
+}
 
-// part[c]: particles and items of the block's cells before c; pre[b]: of the blocks before b,
-// pre[number of blocks]: all.  The counts are cleared for the next binning.
-__global__ void __launch_bounds__(kScanThreads) k_scan(int ncells, int32_t *count, unsigned long long *part,
-                                                       unsigned long long *pre, unsigned *ticket, int log2_homes,
-                                                       int do_tick, int nsims, SimParams *sims, double *red) {
+// part[c]: particles and items of the block's cells before c (the items of four consecutive
+// cells count as the first one's); pre[b]: of the blocks before b, pre[number of blocks]: all.
+// The counts are cleared for the next binning.
+__global__ void __launch_bounds__(kScanThreads) k_scan(int ncells, int32_t *count, const uchar4 *column,
+                                                       unsigned long long *part, unsigned long long *pre,
+                                                       unsigned *ticket, int homes, bool runs, int do_tick, int nsims,
+                                                       SimParams *sims, double *red) {
     step_kernel_begin();
     if (do_tick)
         for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nsims; k += gridDim.x * blockDim.x) tick(sims[k], red);
     const int c = blockIdx.x * kScanCells + 4 * threadIdx.x;
-    int m[4];
-    unsigned long long v = 0;
+    int m[4] = {0, 0, 0, 0};
+    int n4 = 0, items = 0;
+    if (c < ncells) {
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-        m[k] = c + k < ncells ? count[c + k] : 0;
-        v += (unsigned long long)cell_items(m[k], log2_homes) << 32 | (unsigned)m[k];
+        for (int k = 0; k < 4; k++) {
+            m[k] = c + k < ncells ? count[c + k] : 0;
+            n4 += m[k];
+        }
+        if (n4)
+            items = cell_items(m, runs ? column[c / 4] : uchar4(), homes, runs, [](int, int, int, int) {});
     }
-    unsigned long long tot, ex = block_scan2(v, &tot);
+    unsigned long long tot, ex = block_scan2((unsigned long long)items << 32 | (unsigned)n4, &tot);
 #pragma unroll
     for (int k = 0; k < 4; k++)
         if (c + k < ncells) {
             part[c + k] = ex;
             if (m[k]) count[c + k] = 0;
-            ex += (unsigned long long)cell_items(m[k], log2_homes) << 32 | (unsigned)m[k];
+            ex += (unsigned)m[k] + (k == 0 ? (unsigned long long)items << 32 : 0ull);
         }
     __shared__ bool last;
     if (threadIdx.x == 0) {
@@ -303,20 +352,30 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(int ncells, int32_t *coun
     if (threadIdx.x == 0) pre[nb] = all;
 }
 
-__global__ void k_place(int n, int ncells, const int32_t *cell, const int32_t *lidx, const unsigned long long *part,
-                        const unsigned long long *pre, int nb, const float4 *aux, int32_t *start, int2 *items,
-                        int *nitems, int2 *tmp, int log2_homes) {
+__global__ void k_place(int n, int ncells, const int32_t *cell, const int32_t *lidx, const uchar4 *column,
+                        const unsigned long long *part, const unsigned long long *pre, int nb, const float4 *aux,
+                        int32_t *start, int2 *items, int *nitems, int2 *tmp, int homes, bool runs) {
     step_kernel_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < ncells) {
-        const unsigned long long a = part[i] + pre[i / kScanCells];
-        const unsigned long long b = i + 1 < ncells ? part[i + 1] + pre[(i + 1) / kScanCells] : pre[nb];
-        start[i] = (int)(unsigned)a;
-        const int i0 = (int)(a >> 32), i1 = (int)(b >> 32);
-        for (int k = i0; k < i1; k++) items[k] = make_int2(i, (k - i0) << log2_homes);
-        if (i == ncells - 1) {
-            start[ncells] = (int)(unsigned)b;
-            *nitems = i1;
+    auto before = [&](int c) { return c < ncells ? part[c] + pre[c / kScanCells] : pre[nb]; };
+    if (i < ncells) start[i] = (int)(unsigned)before(i);
+    if (i < (ncells + 3) / 4) {   // the items of cells 4 i .. 4 i + 3
+        const int c = 4 * i;
+        const unsigned long long at = before(c);
+        int m[4], p0 = (int)(unsigned)at;
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int p1 = (int)(unsigned)before(min(c + k + 1, ncells));
+            m[k] = p1 - p0;
+            p0 = p1;
+        }
+        int2 *out = items + (at >> 32);
+        cell_items(m, runs ? column[c / 4] : uchar4(), homes, runs, [&](int first, int cells, int c0, int q) {
+            out[q] = make_int2(c + first, c0 | (cells - 1) << 30);
+        });
+        if (i == 0) {
+            start[ncells] = (int)(unsigned)pre[nb];
+            *nitems = (int)(pre[nb] >> 32);
         }
     }
     if (i < n) {
@@ -394,10 +453,12 @@ __global__ void k_rank_scatter(int n, int cap, int nspec, const int2 *tmp, const
 }
 
 // The whole binning of a small arena in one launch, by one cluster of eight blocks.  Four
-// launches take 10 us however few particles there are; this takes two cluster barriers.  Every
-// block scans all counts itself, so the cell starts are in its shared memory.
-constexpr int kSmallBlocks = 8, kSmallThreads = 1024, kSmallPer = 2;   // up to 16,384 particles
-constexpr int kSmallCells = 16 * kSmallThreads;
+// launches take 9 to 13 us however few particles there are; this takes two cluster barriers
+// (7 us for 500 particles, 10 for 8,000; with two particles a thread it was slower than four
+// launches, 16 against 14 us for 11,000).  Every block scans all counts itself, so the cell
+// starts are in its shared memory.
+constexpr int kSmallBlocks = 8, kSmallThreads = 1024;   // one particle each
+constexpr int kSmallCells = 16 * kSmallThreads;   // a multiple of 4 per thread
 
 __device__ __forceinline__ void cluster_barrier() {
     asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
@@ -410,66 +471,62 @@ __global__ void __cluster_dims__(kSmallBlocks, 1, 1) __launch_bounds__(kSmallThr
     stamp_begin(b.stamp);
     const int t0 = blockIdx.x * kSmallThreads + threadIdx.x;
     // count
-    int c[kSmallPer], l[kSmallPer], id[kSmallPer];
-#pragma unroll
-    for (int r = 0; r < kSmallPer; r++) {
-        const int i = t0 + r * kSmallBlocks * kSmallThreads;
-        if (i < b.n) {
-            id[r] = __float_as_int(b.src.aux[i].w);
-            c[r] = recheck(i, b.sims, b.cell_sim, b.src.pos, b.src.cell, b.shuffle);
-            l[r] = atomicAdd(&b.count[c[r]], 1);
-        }
+    int c = 0, l = 0, id = 0;
+    if (t0 < b.n) {
+        id = __float_as_int(b.src.aux[t0].w);
+        c = recheck(t0, b.sims, b.cell_sim, b.src.pos, b.src.cell, b.shuffle);
+        l = atomicAdd(&b.count[c], 1);
     }
     cluster_barrier();
     // scan: thread t holds cells [per t, per (t + 1)); the blocks share the writing
-    const int per = (b.ncells + kSmallThreads - 1) / kSmallThreads, first = per * threadIdx.x;
+    const int per = ((b.ncells + kSmallThreads - 1) / kSmallThreads + 3) & ~3, first = per * threadIdx.x;
+    // (the count array and start_s go on to a multiple of four)
     unsigned long long sum = 0;
-    for (int k = 0; k < per; k++)
-        if (first + k < b.ncells) {
-            const int m = __ldcg(&b.count[first + k]);
-            start_s[first + k] = m;
-            sum += (unsigned long long)cell_items(m, b.log2_homes) << 32 | (unsigned)m;
-        }
+#pragma unroll 1
+    for (int k = first; k < min(first + per, b.ncells); k += 4) {
+        const int4 m4 = __ldcg(reinterpret_cast<const int4 *>(b.count + k));
+        *reinterpret_cast<int4 *>(start_s + k) = m4;
+        const int m[4] = {m4.x, m4.y, m4.z, m4.w}, n4 = m[0] + m[1] + m[2] + m[3];
+        if (n4)
+            sum += (unsigned long long)cell_items(m, b.runs ? b.column[k / 4] : uchar4(), b.homes, b.runs,
+                                                  [](int, int, int, int) {}) << 32 | (unsigned)n4;
+    }
     unsigned long long all, run = block_scan2(sum, &all);
     const bool mine = (threadIdx.x & (kSmallBlocks - 1)) == blockIdx.x;
-    for (int k = 0; k < per; k++)
-        if (first + k < b.ncells) {
-            const int m = start_s[first + k], items = cell_items(m, b.log2_homes);
-            start_s[first + k] = (int)(unsigned)run;
-            if (mine) {
-                b.start[first + k] = (int)(unsigned)run;
-                for (int q = 0; q < items; q++) b.items[(run >> 32) + q] = make_int2(first + k, q << b.log2_homes);
-            }
-            run += (unsigned long long)items << 32 | (unsigned)m;
+#pragma unroll 1
+    for (int k = first; k < min(first + per, b.ncells); k += 4) {
+        const int4 m4 = *reinterpret_cast<const int4 *>(start_s + k);
+        const int m[4] = {m4.x, m4.y, m4.z, m4.w}, n4 = m[0] + m[1] + m[2] + m[3], p = (int)(unsigned)run;
+        const int4 s4 = make_int4(p, p + m[0], p + m[0] + m[1], p + m[0] + m[1] + m[2]);
+        *reinterpret_cast<int4 *>(start_s + k) = s4;
+        if (mine) *reinterpret_cast<int4 *>(b.start + k) = s4;
+        if (n4) {
+            int2 *out = b.items + (run >> 32);
+            run += (unsigned)n4;
+            run += (unsigned long long)cell_items(m, b.runs ? b.column[k / 4] : uchar4(), b.homes, b.runs,
+                                                  [&](int f, int cells, int c0, int q) {
+                                                      if (mine) out[q] = make_int2(k + f, c0 | (cells - 1) << 30);
+                                                  }) << 32;
         }
-    if (t0 == 0) {
-        b.start[b.ncells] = (int)(unsigned)all;
-        *b.nitems = (int)(all >> 32);
     }
+    if (t0 == 0) *b.nitems = (int)(all >> 32);
     if (b.shuffle)
         for (int k = t0; k < b.nsims; k += kSmallBlocks * kSmallThreads) tick(b.sims[k], b.red);
     __syncthreads();
     // place
-#pragma unroll
-    for (int r = 0; r < kSmallPer; r++) {
-        const int i = t0 + r * kSmallBlocks * kSmallThreads;
-        if (i < b.n) b.tmp[start_s[c[r]] + l[r]] = make_int2(id[r], i);
-    }
+    if (t0 < b.n) b.tmp[start_s[c] + l] = make_int2(id, t0);
     cluster_barrier();
+    // (behind the last group's four starts)
+    if (t0 == 0) b.start[b.ncells] = (int)(unsigned)all;
     // the counts return to zero; rank and move
     if (mine)
         for (int k = 0; k < per; k++)
             if (first + k < b.ncells) b.count[first + k] = 0;
-#pragma unroll
-    for (int r = 0; r < kSmallPer; r++) {
-        const int t = t0 + r * kSmallBlocks * kSmallThreads;
-        if (t < b.n) {
-            const int2 me = b.tmp[t];
-            const int cc = b.src.cell[me.y];
-            rank_and_move<kExt, kRand>(me.x, me.y, cc, start_s[cc], cc + 1 < b.ncells ? start_s[cc + 1] : b.n, b.cap,
-                                       b.nspec, b.tmp, b.src, b.dst, b.slot_of_id, b.sims, b.cell_sim, b.rforce, b.force,
-                                       b.oldx);
-        }
+    if (t0 < b.n) {
+        const int2 me = b.tmp[t0];
+        const int cc = b.src.cell[me.y];
+        rank_and_move<kExt, kRand>(me.x, me.y, cc, start_s[cc], cc + 1 < b.ncells ? start_s[cc + 1] : b.n, b.cap, b.nspec,
+                                   b.tmp, b.src, b.dst, b.slot_of_id, b.sims, b.cell_sim, b.rforce, b.force, b.oldx);
     }
 }
 
@@ -865,6 +922,11 @@ inline int nblk(long long n, int t) { return (int)((n + t - 1) / t); }
 
 void launch_stamp(unsigned long long *t, int k, cudaStream_t s) { k_stamp<<<1, 1, 0, s>>>(t, k); }
 
+void launch_fill_cells(int nsims, const SimParams *sims, int32_t *cell_sim, int4 *cell_at, unsigned char *column,
+                       cudaStream_t s) {
+    if (nsims > 0) k_fill_cells<<<dim3(nsims, 32), kThreads, 0, s>>>(sims, cell_sim, cell_at, column);
+}
+
 void launch_setpartp(int n, const float *xg, const SimParams &P, float3 lo, float3 hi, float3 org, float3 ih,
                      int slot0, int32_t *cell, float4 *pos, float4 *aux, const int32_t *type, uint32_t *err,
                      cudaStream_t s) {
@@ -882,22 +944,22 @@ void launch_relocate(int n, int src0, int dst0, int cap_src, int cap_dst, int ns
 int scan_blocks(int ncells) { return nblk(ncells, kScanCells); }
 
 template <bool kExt, bool kRand> void launch_bin_variant(const BinArgs &b, cudaStream_t s) {
-    if (b.n <= kSmallPer * kSmallBlocks * kSmallThreads && b.ncells <= kSmallCells) {
+    if (b.n <= kSmallBlocks * kSmallThreads && b.ncells <= kSmallCells) {
         static const cudaError_t attr = cudaFuncSetAttribute(
             k_bin_small<kExt, kRand>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallCells * (int)sizeof(int32_t));
         (void)attr;   // a failure shows at the launch
-        launch_step_kernel(k_bin_small<kExt, kRand>, kSmallBlocks, kSmallThreads, sizeof(int32_t) * b.ncells, s, b);
+        launch_step_kernel(k_bin_small<kExt, kRand>, kSmallBlocks, kSmallThreads, sizeof(int32_t) * kSmallCells, s, b);
         return;
     }
     if (b.n > 0)
         launch_step_kernel(k_bin_count, nblk(b.n, kThreads), kThreads, 0, s, b.n, b.sims, b.cell_sim, b.src.pos,
                            b.src.cell, b.count, b.lidx, b.shuffle, b.stamp);
     const int nb = scan_blocks(b.ncells);
-    launch_step_kernel(k_scan, nb, kScanThreads, 0, s, b.ncells, b.count, b.part, b.pre, b.ticket, b.log2_homes, b.shuffle,
-                       b.nsims, b.sims, b.red);
+    launch_step_kernel(k_scan, nb, kScanThreads, 0, s, b.ncells, b.count, b.column, b.part, b.pre, b.ticket, b.homes,
+                       b.runs, b.shuffle, b.nsims, b.sims, b.red);
     launch_step_kernel(k_place, nblk(b.n > b.ncells ? b.n : b.ncells, kThreads), kThreads, 0, s, b.n, b.ncells,
-                       b.src.cell, b.lidx, b.part, b.pre, nb, b.src.aux, b.start, b.items, b.nitems, b.tmp,
-                       b.log2_homes);
+                       b.src.cell, b.lidx, b.column, b.part, b.pre, nb, b.src.aux, b.start, b.items, b.nitems, b.tmp,
+                       b.homes, b.runs);
     if (b.n > 0)
         launch_step_kernel(k_rank_scatter<kExt, kRand>, nblk(b.n, kThreads), kThreads, 0, s, b.n, b.cap, b.nspec, b.tmp,
                            b.start, b.src, b.dst, b.slot_of_id, b.sims, b.cell_sim, b.rforce, b.force, b.oldx);

@@ -18,13 +18,15 @@ struct BinArgs {
     double *red;
     const int32_t *cell_sim;
     ParticleArrays src, dst;
-    int32_t *count, *start, *lidx;   // count is zero between binnings
+    int32_t *count, *start, *lidx;   // count (padded to four) is zero between binnings
     int32_t *slot_of_id;             // null: no bonds or angles
     int2 *tmp;                       // (id, slot before) in cell order
     unsigned long long *part, *pre;  // scan scratch: ncells, scan_blocks(ncells) + 1
     unsigned *ticket;
-    int2 *items;                     // the pair pass's work: (cell, first of up to 2^log2_homes home particles)
-    int log2_homes;
+    const uchar4 *column;            // a byte per cell: first cell of a column along z (padded to four)
+    int2 *items;                     // the pair pass's work: (first cell, first of up to `homes` home particles | cells - 1 << 30)
+    int homes;
+    bool runs;                       // an item may span up to four cells
     int *nitems;
     const float4 *rforce;
     float4 *force;
@@ -33,6 +35,8 @@ struct BinArgs {
 };
 
 int scan_blocks(int ncells);
+void launch_fill_cells(int nsims, const SimParams *sims, int32_t *cell_sim, int4 *cell_at, unsigned char *column,
+                       cudaStream_t s);
 // One thread writes the GPU global timer (ns) into t[k].  The phase boundaries of a step are
 // stamped by its kernels where they can be (null: not at all); this is for the others.
 void launch_stamp(unsigned long long *t, int k, cudaStream_t s);
