@@ -928,7 +928,7 @@ int enqueue_step(tfg_engine *eng, bool advance, bool timed) {
     rc = force_pass(eng, true, timed);
     if (rc) return rc;
     if (advance)
-        launch_advance(eng->n, eng->cap, eng->nspec, eng->sims_dev, eng->cell_sim, eng->A[eng->cur], eng->force,
+        launch_advance(eng->n, eng->cap, eng->nspec, (int)eng->order.size(), eng->sims_dev, eng->cell_sim, eng->A[eng->cur], eng->force,
                        eng->type_mass, eng->type_dyn, eng->species_flags, eng->oldx, eng->red, eng->err, eng->stamps,
                        timed ? 1 << 3 | (eng->nb + eng->na == 0) << 2 : 0, s);
     return check_launch(eng);

@@ -54,7 +54,7 @@ void launch_angles(int na, const SimParams *sims, const int32_t *cell_sim, const
                    const float *bblob, const int32_t *slot_of_id, const float4 *pos, const int32_t *cell,
                    float4 *force, double *red, unsigned long long *stamp, cudaStream_t s);
 // stamp_mask: bit k (2, 3) stamps the kernel's begin into stamps[k]; when not 0, its end into stamps[4].
-void launch_advance(int n, int cap, int nspec, SimParams *sims, const int32_t *cell_sim,
+void launch_advance(int n, int cap, int nspec, int nsims, SimParams *sims, const int32_t *cell_sim,
                     const ParticleArrays &A, const float4 *force, const float *type_mass, const int32_t *type_dyn,
                     const uint32_t *species_flags, const float4 *oldx, double *red, uint32_t *err,
                     unsigned long long *stamps, int stamp_mask, cudaStream_t s);
