@@ -1,7 +1,8 @@
 """The binning and the tiled pair pass at the sizes where their launches change: arenas of one
 cluster launch or four (8,192 particles and 16,384 cells), 8, 16 or 32 home particles per
-work item (24,000 and 140,000, with DPD 250,000 particles), partly filled groups, windows and tiles, cells of
-several items; and the graphs of several steps.  Cells and pair sets bit-exact against the
+work item (24,000 and 100,000, with DPD 250,000 particles), runs of cells (450,000 particles),
+partly filled groups, windows and tiles, cells of several items; one potential or several; and
+the graphs of several steps.  Cells and pair sets bit-exact against the
 oracle, forces and densities at its bar."""
 import dataclasses
 
@@ -10,6 +11,7 @@ import pytest
 
 from helpers import FORCE_RTOL, force_error, make_gpu, make_oracle
 from tfg import abi, configs
+from tfg.engine import _potential
 
 pytestmark = pytest.mark.gpu
 
@@ -43,7 +45,8 @@ def _sparse(cells):
 
 
 CASES = {"cells_%d" % n: (lambda n=n: _cells(n)) for n in
-         (1, 2, 31, 33, 97, 1000, 8192, 8193, 16385, 23999, 24000, 139_999, 140_001)}
+         (1, 2, 31, 33, 97, 1000, 8192, 8193, 16385, 23999, 24000, 99_999, 100_001, 139_999,
+          140_001, 449_999, 450_001)}
 CASES.update({"dpd_%d" % n: (lambda n=n: _dpd(n)) for n in (1, 64, 129, 3001, 8192, 16385, 24001, 250_001)})
 CASES.update({"clumps_%d" % n: (lambda n=n: _clumps(n)) for n in (150, 1203, 6000, 26_001)})
 # runs of one to four cells along z per work item: few particles a cell, columns of 3 to 9 cells
@@ -74,6 +77,27 @@ def test_force_pass_at_the_edges(name):
     assert np.array_equal(gc, oc) and np.array_equal(gh, oh)
     assert force_error(a["f"], r["f"], o.fmag()) < FORCE_RTOL
     assert np.abs(a["density"] - r["density"]).max() <= 1e-5 * np.abs(r["density"]).max()
+
+
+def test_potentials_replaced():
+    """Tables, DPD, one table for all types, tables again on one engine: the pair pass reads each
+    set another way, and the table buffers grow under it."""
+    w = _cells(3000)
+    g, o = make_gpu(w), make_oracle(w)
+    spec = list(w.pots.values())
+    dpd = _dpd(8).pots
+    sets = [[next(iter(dpd.values()))] * len(spec), [spec[0]] * len(spec), spec]
+    keep = []
+    for specs in [None] + sets:
+        for e in (g, o):
+            for (ti, tj), q in zip(w.pots, specs or []):
+                keep.append(_potential(q, None, getattr(e, "potential_from_spec", None)))
+                e.set_potential(ti, tj, keep[-1].ptr)
+            e.force_only()
+        a, r = g.download(), o.download()
+        if specs is None or specs[0] not in dpd.values():   # (DPD draws differ)
+            assert force_error(a["f"], r["f"], o.fmag()) < FORCE_RTOL
+        assert np.array_equal(g.pair_signature()[1], o.signature()[1])
 
 
 @pytest.mark.parametrize("n", [500, 16385])

@@ -48,7 +48,7 @@ struct __align__(16) PotDev {
 static_assert(sizeof(PotDev) == 64, "PotDev layout");
 enum : uint32_t { POT_NONE = 0, POT_TABLE = 1, POT_DPD = 2 };
 
-// The same potential as the tiled pair pass reads it, in two 128-bit loads per pair.
+// The same potential as the tiled pair pass reads it.
 struct __align__(16) PotPair {
     float p0, p1, p2, b;   // table: alpha0..2; DPD: alpha, gamma, sigma
     float a, c;            // c: r0_plusone (table), 1/b (DPD)

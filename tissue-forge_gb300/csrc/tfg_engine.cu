@@ -343,6 +343,34 @@ PotPair to_pair(const PotDev &p) {
     return c;
 }
 
+// A table buffer for `need` elements and, when `fetched`, a texture of 16-byte texels over all of
+// it, by which the pair pass on tables reads it; tex stays 0 where the buffer has more texels than
+// a texture can have.
+template <typename T>
+int ensure_fetched(tfg_engine *eng, T **p, size_t &cap, size_t need, bool fetched, cudaTextureObject_t &tex) {
+    const bool kept = need <= cap && *p;
+    const int rc = ensure(eng, p, cap, need);   // (cudaFree waits for the kernels that read the old one)
+    if (!kept && tex) {
+        cudaDestroyTextureObject(tex);
+        tex = 0;
+    }
+    if (rc || !fetched || tex) return rc;
+    cudaResourceDesc res;
+    std::memset(&res, 0, sizeof(res));
+    res.resType = cudaResourceTypeLinear;
+    res.res.linear.devPtr = *p;
+    res.res.linear.desc = cudaCreateChannelDesc<uint4>();
+    res.res.linear.sizeInBytes = cap * sizeof(T);
+    size_t most = 0;
+    CK(cudaDeviceGetTexture1DLinearMaxWidth(&most, &res.res.linear.desc, eng->device));
+    if (cap * sizeof(T) / sizeof(uint4) > most) return TFG_OK;
+    cudaTextureDesc how;
+    std::memset(&how, 0, sizeof(how));
+    how.readMode = cudaReadModeElementType;
+    CK(cudaCreateTextureObject(&tex, &res, &how, nullptr));
+    return TFG_OK;
+}
+
 // Upload the interaction tables of every live simulation (potentials with their table
 // blob, fluxes, per-type arrays, species flags) and the bonded potentials.
 int upload_tables(tfg_engine *eng) {
@@ -415,7 +443,8 @@ int upload_tables(tfg_engine *eng) {
     eng->flags_all = nodens;
     if (blob.empty()) blob.assign(kChunk, 0.f);   // row 0 of no table is readable
     int rc;
-    if ((rc = ensure(eng, &eng->blob, eng->blob_cap, blob.size())) ||
+    const bool tables = !eng->has_dpd && !(eng->has_flux && eng->nspec > 0);   // as launch_pair_tile has it
+    if ((rc = ensure_fetched(eng, &eng->blob, eng->blob_cap, blob.size(), tables, eng->blob_tex)) ||
         (rc = ensure(eng, &eng->pots, eng->pots_cap, pots.size())) ||
         (rc = ensure(eng, &eng->fluxes, eng->fluxes_cap, fl.size())) ||
         (rc = ensure(eng, &eng->species_flags, eng->spec_cap, spf.size())) ||
@@ -423,7 +452,9 @@ int upload_tables(tfg_engine *eng) {
         return rc;
     std::vector<PotPair> pc(pots.size());
     for (size_t k = 0; k < pots.size(); k++) pc[k] = to_pair(pots[k]);
-    if ((rc = ensure(eng, &eng->potc, eng->potc_cap, pc.size()))) return rc;
+    if ((rc = ensure_fetched(eng, &eng->potc, eng->potc_cap, pc.size(), tables, eng->potc_tex))) return rc;
+    eng->one = pc[0];
+    eng->has_one = std::all_of(pc.begin(), pc.end(), [&](const PotPair &c) { return !std::memcmp(&c, &pc[0], sizeof(c)); });
     CK(cudaMemcpyAsync(eng->potc, pc.data(), sizeof(PotPair) * pc.size(), cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(eng->wpots, wp.data(), sizeof(PotDev) * wp.size(), cudaMemcpyHostToDevice, s));
     if (rf.size() > eng->types_cap) {
@@ -860,6 +891,10 @@ PairKernelArgs pair_args(tfg_engine *eng) {
     a.potc = eng->potc;
     a.blob = eng->blob;
     a.blob_floats = eng->blob_floats;
+    a.potc_tex = eng->potc_tex;
+    a.blob_tex = eng->blob_tex;
+    a.one = eng->one;
+    a.has_one = eng->has_one;
     a.fluxes = eng->fluxes;
     a.wpots = eng->wpots;
     a.has_wall_pots = eng->has_wall_pots;
@@ -1206,6 +1241,8 @@ void destroy(tfg_engine *eng) {
                     eng->sims_dev, eng->corig, eng->pots, eng->potc, eng->blob, eng->fluxes, eng->rforce, eng->type_mass,
                     eng->type_dyn, eng->species_flags, eng->bonds, eng->bond_slot, eng->angles, eng->bpots,
                     eng->bblob, eng->red, eng->err, eng->oldx, eng->stage};
+    for (cudaTextureObject_t t : {eng->potc_tex, eng->blob_tex})
+        if (t) cudaDestroyTextureObject(t);
     for (void *p : bufs) cudaFree(p);
     for (int k = 0; k < 5; k++)
         if (eng->ev[k]) cudaEventDestroy(eng->ev[k]);

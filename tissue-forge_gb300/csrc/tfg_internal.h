@@ -85,6 +85,9 @@ struct PairKernelArgs {
     const PotDev *pots;         // nsims * max_type^2
     const PotPair *potc;        // the same, compact (tiled pass)
     const float *blob;
+    cudaTextureObject_t potc_tex, blob_tex;   // potc and blob as textures of 16 bytes a texel, or 0
+    PotPair one;                // the entry that all of potc's are equal to
+    bool has_one;               // there is one
     int blob_floats;
     const PotDev *wpots;        // nsims * 6 * max_type wall potentials
     bool has_wall_pots;         // any simulation has a wall potential
