@@ -454,7 +454,9 @@ int upload_tables(tfg_engine *eng) {
     for (size_t k = 0; k < pots.size(); k++) pc[k] = to_pair(pots[k]);
     if ((rc = ensure_fetched(eng, &eng->potc, eng->potc_cap, pc.size(), tables, eng->potc_tex))) return rc;
     eng->one = pc[0];
-    eng->has_one = std::all_of(pc.begin(), pc.end(), [&](const PotPair &c) { return !std::memcmp(&c, &pc[0], sizeof(c)); });
+    eng->one_flux = fl[0];
+    eng->has_one = std::all_of(pc.begin(), pc.end(), [&](const PotPair &c) { return !std::memcmp(&c, &pc[0], sizeof(c)); }) &&
+                   std::all_of(fl.begin(), fl.end(), [&](const FluxSet &f) { return !std::memcmp(&f, &fl[0], sizeof(f)); });
     CK(cudaMemcpyAsync(eng->potc, pc.data(), sizeof(PotPair) * pc.size(), cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(eng->wpots, wp.data(), sizeof(PotDev) * wp.size(), cudaMemcpyHostToDevice, s));
     if (rf.size() > eng->types_cap) {
@@ -894,6 +896,7 @@ PairKernelArgs pair_args(tfg_engine *eng) {
     a.potc_tex = eng->potc_tex;
     a.blob_tex = eng->blob_tex;
     a.one = eng->one;
+    a.one_flux = eng->one_flux;
     a.has_one = eng->has_one;
     a.fluxes = eng->fluxes;
     a.wpots = eng->wpots;

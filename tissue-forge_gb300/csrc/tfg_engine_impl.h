@@ -87,8 +87,9 @@ struct tfg_engine {
     tfg::PotPair *potc = nullptr;     // the same in the tiled pair pass's compact form
     size_t potc_cap = 0;
     cudaTextureObject_t potc_tex = 0, blob_tex = 0;   // potc and blob, for the pair pass on tables
-    tfg::PotPair one;                 // the one potential of all type pairs
-    bool has_one = false;             // there is one
+    tfg::PotPair one;                 // the one potential and the one set of fluxes of all type pairs
+    tfg::FluxSet one_flux;
+    bool has_one = false;             // there are such
     float *blob = nullptr;
     size_t blob_cap = 0;
     int blob_floats = 0;

@@ -86,8 +86,9 @@ struct PairKernelArgs {
     const PotPair *potc;        // the same, compact (tiled pass)
     const float *blob;
     cudaTextureObject_t potc_tex, blob_tex;   // potc and blob as textures of 16 bytes a texel, or 0
-    PotPair one;                // the entry that all of potc's are equal to
-    bool has_one;               // there is one
+    PotPair one;                // the entries that all of potc's and fluxes' are equal to
+    FluxSet one_flux;
+    bool has_one;               // there are such
     int blob_floats;
     const PotDev *wpots;        // nsims * 6 * max_type wall potentials
     bool has_wall_pots;         // any simulation has a wall potential
