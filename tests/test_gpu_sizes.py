@@ -1,9 +1,8 @@
 """The binning and the tiled pair pass at the sizes where their launches change: arenas of one
-cluster launch or four (8,192 particles and 16,384 cells), 8, 16 or 32 home particles per
-work item (24,000 and 100,000, with DPD 250,000 particles), runs of cells (450,000 particles),
-partly filled groups, windows and tiles, cells of several items; one potential or several; and
-the graphs of several steps.  Cells and pair sets bit-exact against the
-oracle, forces and densities at its bar."""
+cluster launch or four (8,192 particles and 16,384 cells), 8, 16 or 32 home particles per work
+item (24,000 and 110,000 particles), runs of cells (400,000 particles), partly filled groups,
+windows and tiles, cells of several items; one potential or several; and the graphs of several
+steps. Cells and pair sets bit-exact against the oracle, forces and densities at its bar."""
 import dataclasses
 
 import numpy as np
@@ -45,8 +44,8 @@ def _sparse(cells):
 
 
 CASES = {"cells_%d" % n: (lambda n=n: _cells(n)) for n in
-         (1, 2, 31, 33, 97, 1000, 8192, 8193, 16385, 23999, 24000, 99_999, 100_001, 139_999,
-          140_001, 449_999, 450_001)}
+         (1, 2, 31, 33, 97, 1000, 8192, 8193, 16385, 23999, 24000, 109_999, 110_001, 399_999,
+          400_001)}
 CASES.update({"dpd_%d" % n: (lambda n=n: _dpd(n)) for n in (1, 64, 129, 3001, 8192, 16385, 24001, 250_001)})
 CASES.update({"clumps_%d" % n: (lambda n=n: _clumps(n)) for n in (150, 1203, 6000, 26_001)})
 # runs of one to four cells along z per work item: few particles a cell, columns of 3 to 9 cells

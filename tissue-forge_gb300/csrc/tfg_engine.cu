@@ -794,17 +794,19 @@ int load_sim(tfg_engine *eng, int sim, int n, const float *xg, const int32_t *ce
 // Work items of the tiled pass: the most home particles of one, and whether one may span several
 // cells.  A small arena leaves warps without an item, and its time is that of the longest one,
 // a crowded cell's: with 8, 16 and 32 home particles the pass takes 12, 14 and 20 us on 2,000
-// clustered cells, 20, 22 and 32 on 20,000.  Larger items share more: 163, 133 and 120 us on
-// 300,000 uniform cells.  DPD pairs cost more each, so balance counts for longer: 58, 56 and
-// 62 us on 100,000 particles, 136 and 128 (16, 32) on 300,000.
+// clustered cells, 20, 22 and 32 on 20,000.  Larger items share more: the step takes 89, 81 and
+// 86 us on 100,000 uniform cells, 106, 96 and 97 on 150,000, 117 and 115 (16, 32) on 200,000,
+// 150 and 141 on 300,000; 73 and 72 (16, 32) on an LJ fluid of 110,592.  DPD pairs cost more each and droplets spread out, so that balance
+// counts at every size: 82, 77 and 81 us on 100,000 particles, 161 and 173 on 300,000, 967 and
+// 1007 on 2,000,000.
 // Runs of cells share set-up and targets, most where cells hold few particles (DPD droplets
-// that have spread out: 77 -> 38 us), but leave fewer items: on 150,001 uniform cells 67 us
-// without them and 73 with, on
-// 300,000 118 and 121; on LJ fluids of 512,000 and 1,000,000 particles 183 and 180, 351 and 337.
+// that have spread out: 77 -> 38 us), but leave fewer items: without and with them 141 and 144 us
+// on 300,000 uniform cells, 185 and 179 on 400,000; 147 and 151 on LJ fluids of 343,000
+// particles, 178 and 174 on 421,875.
 static void plan_items(tfg_engine *eng) {
     const bool pairs_cost = eng->has_dpd || (eng->has_flux && eng->nspec > 0);
-    eng->homes = eng->n < 24000 ? 8 : (eng->n < (pairs_cost ? 250000 : 100000) ? 16 : 32);
-    eng->runs = pairs_cost || eng->n >= 450000;
+    eng->homes = eng->n < 24000 ? 8 : (pairs_cost || eng->n < 110000 ? 16 : 32);
+    eng->runs = pairs_cost || eng->n >= 400000;
 }
 
 int bin(tfg_engine *eng, int shuffle, bool timed) {
