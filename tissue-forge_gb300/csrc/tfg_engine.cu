@@ -796,9 +796,9 @@ int load_sim(tfg_engine *eng, int sim, int n, const float *xg, const int32_t *ce
 // a crowded cell's: with 8, 16 and 32 home particles the pass takes 12, 14 and 20 us on 2,000
 // clustered cells, 20, 22 and 32 on 20,000.  Larger items share more: the step takes 89, 81 and
 // 86 us on 100,000 uniform cells, 106, 96 and 97 on 150,000, 117 and 115 (16, 32) on 200,000,
-// 150 and 141 on 300,000; 73 and 72 (16, 32) on an LJ fluid of 110,592.  DPD pairs cost more each and droplets spread out, so that balance
-// counts at every size: 82, 77 and 81 us on 100,000 particles, 161 and 173 on 300,000, 967 and
-// 1007 on 2,000,000.
+// 150 and 141 on 300,000; 73 and 72 on an LJ fluid of 110,592.  DPD pairs cost more each and
+// droplets spread out, so that balance counts at every size: 82, 77 and 81 us on 100,000
+// particles, 161 and 173 on 300,000, 967 and 1007 on 2,000,000.
 // Runs of cells share set-up and targets, most where cells hold few particles (DPD droplets
 // that have spread out: 77 -> 38 us), but leave fewer items: without and with them 141 and 144 us
 // on 300,000 uniform cells, 185 and 179 on 400,000; 147 and 151 on LJ fluids of 343,000
