@@ -50,6 +50,8 @@ CASES.update({"dpd_%d" % n: (lambda n=n: _dpd(n)) for n in (1, 64, 129, 3001, 81
 CASES.update({"clumps_%d" % n: (lambda n=n: _clumps(n)) for n in (150, 1203, 6000, 26_001)})
 # runs of one to four cells along z per work item: few particles a cell, columns of 3 to 9 cells
 CASES.update({"thin_%d" % k: (lambda k=k: _thin(k)) for k in (3, 4, 5, 6, 7, 9)})
+# one bond or angle to a thread and several
+CASES.update({"bonded_%d" % n: (lambda n=n: configs.bonded_fluid(n=n, seed=9)) for n in (16 * 99, 16 * 17_000)})
 CASES.update({"grid_%dx%dx%d" % c: (lambda c=c: _sparse(c)) for c in ((3, 3, 1820), (3, 3, 1821))})
 
 

@@ -931,9 +931,9 @@ int force_pass(tfg_engine *eng, bool bonded, bool timed) {
         }
     }
     if (bonded) {
-        launch_bonds(eng->nb, eng->sims_dev, eng->cell_sim, eng->bonds, eng->bond_slot, eng->bpots, eng->bblob,
+        launch_bonds(eng->nb, eng->sms, eng->sims_dev, eng->cell_sim, eng->bonds, eng->bond_slot, eng->bpots, eng->bblob,
                      eng->slot_of_id, A.pos, A.aux, A.cell, eng->force, eng->red, timed ? eng->stamps + 2 : nullptr, s);
-        launch_angles(eng->na, eng->sims_dev, eng->cell_sim, eng->angles, eng->bpots, eng->bblob, eng->slot_of_id,
+        launch_angles(eng->na, eng->sms, eng->sims_dev, eng->cell_sim, eng->angles, eng->bpots, eng->bblob, eng->slot_of_id,
                       A.pos, A.cell, eng->force, eng->red, timed && eng->nb == 0 ? eng->stamps + 2 : nullptr, s);
     }
     return check_launch(eng);

@@ -21,11 +21,11 @@ __device__ __forceinline__ int sim_of(int nsims, const int32_t *cell_sim, int c)
 
 __device__ __forceinline__ int wrap_shift(int s) { return s > 1 ? -1 : (s < -1 ? 1 : s); }
 
-// Add per-thread FP32 partials into per-simulation FP64 totals.  When the whole block
-// belongs to one simulation: FP32 over each warp, FP64 across warps, one atomic per
-// block.  Otherwise each warp whose lanes share a simulation adds once, and mixed warps
+// Add per-thread partials (FP32, or FP64 of several terms) into per-simulation FP64 totals.  When
+// the whole block belongs to one simulation: the partials' type over each warp, FP64 across
+// warps, one atomic per block.  Otherwise each warp whose lanes share a simulation adds once, and mixed warps
 // add lane by lane.  Every thread of the block must call it.
-__device__ __forceinline__ void keyed_add(double *red, int rb, int slot, float v) {
+template <class T> __device__ __forceinline__ void keyed_add(double *red, int rb, int slot, T v) {
     __shared__ double part[32];
     const int rb0 = __shfl_sync(0xffffffffu, rb, 0);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
@@ -34,7 +34,7 @@ __device__ __forceinline__ void keyed_add(double *red, int rb, int slot, float v
     __syncthreads();
     const bool uniform = __syncthreads_and(rb == block_rb || rb < 0);
     if (uniform) {
-        float s = v;
+        T s = v;
         for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
         if (lane == 0) part[w] = (double)s;
         __syncthreads();
@@ -47,17 +47,18 @@ __device__ __forceinline__ void keyed_add(double *red, int rb, int slot, float v
         return;
     }
     if (__all_sync(0xffffffffu, rb == rb0 || rb < 0)) {
-        float s = v;
+        T s = v;
         for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-        if (lane == 0 && rb0 >= 0 && s != 0.f) atomicAdd(&red[rb0 + slot], (double)s);
-    } else if (rb >= 0 && v != 0.f) {
+        if (lane == 0 && rb0 >= 0 && s != T(0)) atomicAdd(&red[rb0 + slot], (double)s);
+    } else if (rb >= 0 && v != T(0)) {
         atomicAdd(&red[rb + slot], (double)v);
     }
 }
 
 // keyed_add of three values to three slots of the same simulation, under one set of block
 // barriers.
-__device__ __forceinline__ void keyed_add3(double *red, int rb, int s0, float v0, int s1, float v1, int s2, float v2) {
+template <class T>
+__device__ __forceinline__ void keyed_add3(double *red, int rb, int s0, T v0, int s1, T v1, int s2, T v2) {
     __shared__ double part3[3][32];
     const int rb0 = __shfl_sync(0xffffffffu, rb, 0);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
@@ -65,7 +66,7 @@ __device__ __forceinline__ void keyed_add3(double *red, int rb, int s0, float v0
     if (threadIdx.x == 0) block_rb3 = rb;
     __syncthreads();
     const bool uniform = __syncthreads_and(rb == block_rb3 || rb < 0);
-    float a = v0, b = v1, c = v2;
+    T a = v0, b = v1, c = v2;
     if (uniform || __all_sync(0xffffffffu, rb == rb0 || rb < 0)) {
         for (int o = 16; o > 0; o >>= 1) {
             a += __shfl_down_sync(0xffffffffu, a, o);
@@ -91,14 +92,14 @@ __device__ __forceinline__ void keyed_add3(double *red, int rb, int s0, float v0
     }
     if (__all_sync(0xffffffffu, rb == rb0 || rb < 0)) {
         if (lane == 0 && rb0 >= 0) {
-            if (a != 0.f) atomicAdd(&red[rb0 + s0], (double)a);
-            if (b != 0.f) atomicAdd(&red[rb0 + s1], (double)b);
-            if (c != 0.f) atomicAdd(&red[rb0 + s2], (double)c);
+            if (a != T(0)) atomicAdd(&red[rb0 + s0], (double)a);
+            if (b != T(0)) atomicAdd(&red[rb0 + s1], (double)b);
+            if (c != T(0)) atomicAdd(&red[rb0 + s2], (double)c);
         }
     } else if (rb >= 0) {
-        if (v0 != 0.f) atomicAdd(&red[rb + s0], (double)v0);
-        if (v1 != 0.f) atomicAdd(&red[rb + s1], (double)v1);
-        if (v2 != 0.f) atomicAdd(&red[rb + s2], (double)v2);
+        if (v0 != T(0)) atomicAdd(&red[rb + s0], (double)v0);
+        if (v1 != T(0)) atomicAdd(&red[rb + s1], (double)v1);
+        if (v2 != T(0)) atomicAdd(&red[rb + s2], (double)v2);
     }
 }
 
@@ -544,17 +545,38 @@ __global__ void __cluster_dims__(kSmallBlocks, 1, 1) __launch_bounds__(kSmallThr
     }
 }
 
-// bond_eval (tfBond.cpp:97-345) for table potentials; one thread per bond.
-__global__ void k_bonds(int nb, const SimParams *sims, const int32_t *cell_sim, const int2 *bonds,
+// A thread's sums over its bonds or angles, in FP64, for one simulation at a time.
+struct BondSums {
+    int rb = -1;
+    double epot = 0.0, vir = 0.0;
+    __device__ __forceinline__ void add(double *red, int slot, int to, float e, float v) {
+        if (to != rb) {
+            if (rb >= 0) {
+                atomicAdd(&red[rb + slot], epot);
+                atomicAdd(&red[rb + RED_VIRIAL], vir);
+            }
+            rb = to;
+            epot = vir = 0.0;
+        }
+        epot += e;
+        vir += v;
+    }
+};
+
+// bond_eval (tfBond.cpp:97-345) for table potentials.  Bound by the latency of the gathers by id.  A
+// block takes `per` bonds in a row, so that all blocks are resident at once and their atomics to
+// the simulation's totals, which are serial, are few: with k_angles 93 -> 83 us on 1.9M bonds and
+// 1.8M angles (six blocks per SM; 91 with five, 100 with eight, which are not all resident).
+__global__ void k_bonds(int nb, int per, const SimParams *sims, const int32_t *cell_sim, const int2 *bonds,
                         const int32_t *bslot, const PotDev *bpots, const float *bblob, const int32_t *slot_of_id,
                         const float4 *pos, const float4 *aux, const int32_t *cell, float4 *force, double *red,
                         unsigned long long *stamp) {
     step_kernel_begin();
     stamp_begin(stamp);
-    int b = blockIdx.x * blockDim.x + threadIdx.x;
-    float epot = 0.f, vir = 0.f;
-    int rb = -1;
-    if (b < nb) {
+    BondSums sums;
+    const int last = min(nb, ((int)blockIdx.x + 1) * per);
+#pragma unroll 1
+    for (int b = blockIdx.x * per + threadIdx.x; b < last; b += blockDim.x) {
         const int2 bd = bonds[b];
         const PotDev &pot = bpots[bslot[b]];
         const int si = slot_of_id[bd.x], sj = slot_of_id[bd.y];
@@ -569,7 +591,7 @@ __global__ void k_bonds(int nb, const SimParams *sims, const int32_t *cell_sim, 
         }
         const SimParams &P = sims[cell_sim[ci]];
         if (there && !P.stopped) {
-            rb = P.red_base;
+            float epot = 0.f, vir = 0.f;
             int s0 = 0, s1 = 0, s2 = 0;
             if (ci != cj) {
                 int ai, bi, ki, aj, bj, kj;
@@ -605,21 +627,22 @@ __global__ void k_bonds(int nb, const SimParams *sims, const int32_t *cell_sim, 
                 epot = ee;
                 vir = -f * r2;
             }
+            sums.add(red, RED_EPOT_BOND, P.red_base, epot, vir);
         }
     }
-    keyed_add3(red, rb, RED_EPOT_BOND, epot, RED_VIRIAL, vir, RED_VIRIAL, 0.f);
+    keyed_add3(red, sums.rb, RED_EPOT_BOND, sums.epot, RED_VIRIAL, sums.vir, RED_VIRIAL, 0.0);
 }
 
-// angle_eval (tfAngle.cpp:90-382); one thread per angle, j is the vertex.
-__global__ void k_angles(int na, const SimParams *sims, const int32_t *cell_sim, const int4 *angles,
+// angle_eval (tfAngle.cpp:90-382), j is the vertex; blocks as those of k_bonds.
+__global__ void k_angles(int na, int per, const SimParams *sims, const int32_t *cell_sim, const int4 *angles,
                          const PotDev *bpots, const float *bblob, const int32_t *slot_of_id, const float4 *pos,
                          const int32_t *cell, float4 *force, double *red, unsigned long long *stamp) {
     step_kernel_begin();
     stamp_begin(stamp);
-    int q = blockIdx.x * blockDim.x + threadIdx.x;
-    float epot = 0.f;
-    int rb = -1;
-    if (q < na) {
+    BondSums sums;
+    const int last = min(na, ((int)blockIdx.x + 1) * per);
+#pragma unroll 1
+    for (int q = blockIdx.x * per + threadIdx.x; q < last; q += blockDim.x) {
         const int4 A = angles[q];
         const PotDev &pot = bpots[A.w];
         const int si = slot_of_id[A.x], sj = slot_of_id[A.y], sk = slot_of_id[A.z];
@@ -636,7 +659,7 @@ __global__ void k_angles(int na, const SimParams *sims, const int32_t *cell_sim,
         }
         const SimParams &P = sims[cell_sim[cj]];
         if (there && !P.stopped) {
-            rb = P.red_base;
+            float epot = 0.f;
             int li[3], lj[3], lk[3];
             cell_loc(P, ci, li[0], li[1], li[2]);
             cell_loc(P, cj, lj[0], lj[1], lj[2]);
@@ -692,9 +715,10 @@ __global__ void k_angles(int na, const SimParams *sims, const int32_t *cell_sim,
                     epot = ee;
                 }
             }
+            sums.add(red, RED_EPOT_ANGLE, P.red_base, epot, 0.f);
         }
     }
-    keyed_add(red, rb, RED_EPOT_ANGLE, epot);
+    keyed_add(red, sums.rb, RED_EPOT_ANGLE, sums.epot);
 }
 
 // Verlet mode: the integrator branch of engine_advance_forward_euler for Verlet lists
@@ -1015,20 +1039,23 @@ void launch_bin(const BinArgs &b, cudaStream_t s) {
     else launch_bin_variant<false, false>(b, s);
 }
 
-void launch_bonds(int nb, const SimParams *sims, const int32_t *cell_sim, const int2 *bonds, const int32_t *bslot,
+// Bonds or angles of a block: a multiple of its threads, for at most six blocks per SM.
+static int per_block(int n, int sms) { return nblk(nblk(n, 6 * sms), kThreads) * kThreads; }
+
+void launch_bonds(int nb, int sms, const SimParams *sims, const int32_t *cell_sim, const int2 *bonds, const int32_t *bslot,
                   const PotDev *bpots, const float *bblob, const int32_t *slot_of_id, const float4 *pos,
                   const float4 *aux, const int32_t *cell, float4 *force, double *red, unsigned long long *stamp,
                   cudaStream_t s) {
     if (nb > 0)
-        launch_step_kernel(k_bonds, nblk(nb, kThreads), kThreads, 0, s, nb, sims, cell_sim, bonds, bslot, bpots, bblob,
+        launch_step_kernel(k_bonds, nblk(nb, per_block(nb, sms)), kThreads, 0, s, nb, per_block(nb, sms), sims, cell_sim, bonds, bslot, bpots, bblob,
                            slot_of_id, pos, aux, cell, force, red, stamp);
 }
 
-void launch_angles(int na, const SimParams *sims, const int32_t *cell_sim, const int4 *angles, const PotDev *bpots,
+void launch_angles(int na, int sms, const SimParams *sims, const int32_t *cell_sim, const int4 *angles, const PotDev *bpots,
                    const float *bblob, const int32_t *slot_of_id, const float4 *pos, const int32_t *cell,
                    float4 *force, double *red, unsigned long long *stamp, cudaStream_t s) {
     if (na > 0)
-        launch_step_kernel(k_angles, nblk(na, kThreads), kThreads, 0, s, na, sims, cell_sim, angles, bpots, bblob,
+        launch_step_kernel(k_angles, nblk(na, per_block(na, sms)), kThreads, 0, s, na, per_block(na, sms), sims, cell_sim, angles, bpots, bblob,
                            slot_of_id, pos, cell, force, red, stamp);
 }
 

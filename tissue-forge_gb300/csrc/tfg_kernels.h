@@ -46,11 +46,11 @@ void launch_setpartp(int n, const float *xg, const SimParams &P, float3 lo, floa
 void launch_relocate(int n, int src0, int dst0, int cap_src, int cap_dst, int nspec, int did, int dcell,
                      const ParticleArrays &src, const ParticleArrays &dst, cudaStream_t s);
 void launch_bin(const BinArgs &b, cudaStream_t s);
-void launch_bonds(int nb, const SimParams *sims, const int32_t *cell_sim, const int2 *bonds, const int32_t *bslot,
+void launch_bonds(int nb, int sms, const SimParams *sims, const int32_t *cell_sim, const int2 *bonds, const int32_t *bslot,
                   const PotDev *bpots, const float *bblob, const int32_t *slot_of_id, const float4 *pos,
                   const float4 *aux, const int32_t *cell, float4 *force, double *red, unsigned long long *stamp,
                   cudaStream_t s);
-void launch_angles(int na, const SimParams *sims, const int32_t *cell_sim, const int4 *angles, const PotDev *bpots,
+void launch_angles(int na, int sms, const SimParams *sims, const int32_t *cell_sim, const int4 *angles, const PotDev *bpots,
                    const float *bblob, const int32_t *slot_of_id, const float4 *pos, const int32_t *cell,
                    float4 *force, double *red, unsigned long long *stamp, cudaStream_t s);
 // stamp_mask: bit k (2, 3) stamps the kernel's begin into stamps[k]; when not 0, its end into stamps[4].
