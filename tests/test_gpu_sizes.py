@@ -101,6 +101,33 @@ def test_potentials_replaced():
         assert np.array_equal(g.pair_signature()[1], o.signature()[1])
 
 
+@pytest.mark.parametrize("name", ["dpd", "cells"])
+def test_signature_after_a_step(name):
+    """The pair set of a state that was advanced but not binned again: cells as binned before the
+    step, positions after it, also for particles that have left their cell."""
+    w = _dpd(3001, ref=False) if name == "dpd" else _cells(3001)
+    g = make_gpu(w)
+    g.step(30)
+    c0 = g.download()["cell"].astype(np.int64)
+    g.step(1)
+    d = g.download()
+    assert (d["cell"] != c0).any()
+    dims = np.array(w.cells)
+    loc = np.stack([c0 // (dims[1] * dims[2]), c0 // dims[2] % dims[1], c0 % dims[2]], axis=1)
+    h = np.array(w.dim, np.float64) / dims
+    count, _ = g.pair_signature()
+    x = d["xrel"].astype(np.float64)
+    low, high = np.zeros(w.n, int), np.zeros(w.n, int)
+    for i in range(w.n):
+        off = loc - loc[i]
+        off -= dims * np.rint(off / dims).astype(np.int64)
+        r = np.sqrt((((x - x[i]) + off * h) ** 2).sum(axis=1))
+        near = (np.abs(off) <= 1).all(axis=1)
+        near[i] = False
+        low[i], high[i] = (near & (r < w.cutoff * (1 - 1e-5))).sum(), (near & (r < w.cutoff * (1 + 1e-5))).sum()
+    assert (low <= count).all() and (count <= high).all()
+
+
 @pytest.mark.parametrize("n", [500, 16385])
 def test_steps_in_graphs_of_several(n):
     """One call of 45 steps (single and several-step graphs) and 45 calls give the same bits in
