@@ -62,7 +62,7 @@ WORKLOADS = {
     "lj_fluid": dict(desc="LJ 12-6 fluid from a jittered lattice: 2,000,376 particles at density 0.85, cutoff 2.5, "
                           "T 0.5, dt 0.002, cell lists (cell edge >= cutoff)", bytes_per_particle=64),
     "lj_fluid_verlet": dict(desc="the lj_fluid workload in Verlet mode (engine_flag_verlet): cell edge >= 1.2 cutoff, "
-                                 "re-binning only when 2 maxdx > skin, device pair lists between rebuilds",
+                                 "re-binning only when 2 maxdx > skin",
                             bytes_per_particle=64),
 }
 
@@ -226,16 +226,17 @@ def fp32_peak(dev):
 
 
 # DRAM traffic of the tiled pair kernel per particle of the arena: one ncu capture of the
-# 256-simulation ensemble pass (2,902,298 particles) read 141.3 MB and wrote 26.7 MB
+# 256-simulation ensemble pass (2,902,298 particles; an earlier form of the kernel, which staged
+# the same data) read 141.3 MB and wrote 26.7 MB
 # (dram__bytes_read.sum + dram__bytes_write.sum), 57.9 B per particle.  The traffic is the
 # particle data read and the forces written, so it scales with the particles, not the pairs.
 PAIR_TRAFFIC_BYTES_PER_PARTICLE = 57.9
 
 
-def launches_per_step(has_bonds=False, has_angles=False):
-    # tick, 7 binning kernels (count, 3 scan passes, place, rank, scatter), the tiled pair
-    # kernel and its overflow kernel, bonds, angles, advance
-    return 1 + 7 + 2 + int(has_bonds) + int(has_angles) + 1
+def launches_per_step(n, cells, has_bonds=False, has_angles=False):
+    # binning (count, scan, place, rank and scatter; one cluster launch for small arenas), the
+    # tiled pair kernel, bonds, angles, advance
+    return (1 if n <= 8192 and cells <= 16384 else 4) + 1 + int(has_bonds) + int(has_angles) + 1
 
 
 def ensemble_sample(ws, count):
@@ -591,7 +592,7 @@ def run_ensemble(args, rank, world, dev, dist):
             "plain_gpu": plain, "batched_over_plain": value / plain["value"],
             "serving": serving, "workloads": workloads,
             "roofline": roof, "cpu_baseline": cpu, "e2e": e2e, "clocks": clk.summary(),
-            "gpu_launches": launches_per_step() * args.steps,
+            "gpu_launches": launches_per_step(n_tot, 1 << 30) * args.steps,
         }
         print(json.dumps(line), flush=True)
 
@@ -606,7 +607,7 @@ def tune(eng, args):
 
 
 def pair_kernel_name(split):
-    return "k_pair_home" if split == 32 else "k_pair_tile (split %d)" % split
+    return "k_pair_tile (split %d)" % split
 
 
 def measure_workload(name, dev, stream, steps, warmup, args=None):
@@ -763,20 +764,18 @@ def run_single(args, rank, world, dev, dist):
             "step_hbm": {"achieved_gbs": bytes_alg / (step_ms * 1e-3) / 1e9, "peak_gbs": hbm, "peak_source": hbm_src,
                          "frac": bytes_alg / (step_ms * 1e-3) / 1e9 / hbm, "bytes_per_step": bytes_alg}}
     verlet = None
-    if w.flags & 4:   # Verlet mode: the same fluid with cell lists, and Verlet without pair lists
+    if w.flags & 4:   # Verlet mode: the same fluid with cell lists
         rb_timed = rebuilds1 - rebuilds0
         wc = make_workload("lj_fluid", rank, args.n or None)
         cmp = {}
-        for label, ww, lists in (("cell_lists", wc, True), ("verlet_without_pair_lists", w, False)):
-            e = Engine(ww.desc(device=dev))
-            k = setup_model(e, ww)
-            e.set_stream(stream.cuda_stream)
-            e.set_pair_lists(lists)
-            cmp[label] = timed_rate(e, ww.n, args.steps, args.warmup, flush, stream, world)
-            del e, k
+        e = Engine(wc.desc(device=dev))
+        k = setup_model(e, wc)
+        e.set_stream(stream.cuda_stream)
+        cmp["cell_lists"] = timed_rate(e, wc.n, args.steps, args.warmup, flush, stream, world)
+        del e, k
         verlet = {"skin": float(min(d / c for d, c in zip(w.dim, w.cells)) - w.cutoff),
                   "rebuilds_in_timed_steps": rb_timed, "steps": args.steps,
-                  "cell_lists_value": cmp["cell_lists"], "verlet_without_pair_lists_value": cmp["verlet_without_pair_lists"],
+                  "cell_lists_value": cmp["cell_lists"],
                   "speedup_over_cell_lists": value / cmp["cell_lists"],
                   "how": "same fluid, same steps and L2 flush; cell lists at cell edge >= cutoff"}
     cpu = None
@@ -797,7 +796,8 @@ def run_single(args, rank, world, dev, dist):
                        "phase_ms_per_step": dict(zip(["bin", "pair", "bonded", "advance"],
                                                      (phase_tot / args.steps).round(5).tolist()))},
             "roofline": roof, "cpu_baseline": cpu, "e2e": e2e, "clocks": clk.summary(),
-            "gpu_launches": launches_per_step(w.bonds is not None, w.angles is not None) * args.steps,
+            "gpu_launches": launches_per_step(w.n, int(np.prod(w.cells)), w.bonds is not None,
+                                              w.angles is not None) * args.steps,
         }
         if verlet:
             line["verlet"] = verlet

@@ -288,7 +288,7 @@ TFG_API int tfg_sync(tfg_engine *eng);
 TFG_API int tfg_query(tfg_engine *eng, int *idle);
 /* Replay steps from CUDA graphs (default on): after any change of layout, tables, work
  * split or stream one step runs eagerly, and the following steps replay a captured
- * single-step graph (one per particle-buffer parity), phase events included. */
+ * graph of one step or of several (one per particle-buffer parity), phase stamps included. */
 TFG_API int tfg_set_graphs(tfg_engine *eng, int enable);
 /* Accepted for callers that switch pair lists of simulations in Verlet mode on or off; has no
  * effect: every step tests the candidate pairs of the cell stencil, which is faster than
@@ -296,7 +296,7 @@ TFG_API int tfg_set_graphs(tfg_engine *eng, int enable);
 TFG_API int tfg_set_pair_lists(tfg_engine *eng, int enable);
 /* Autotune the nonbonded pass's form by timing each choice on the current state; the
  * state is left unchanged.  The choices are the tiled kernel's work split (warps per home
- * cell: 1, 2, 7 or 14), its warps per CTA and its smallest grab of work items.  tfg_step and
+ * cell: 1, 2, 7 or 14).  tfg_step and
  * tfg_force_only run it on their first call, and time the work splits again whenever the
  * particle count has grown or shrunk more than 4x since (a batch that fills up or drains);
  * tfg_set_split fixes the choice instead (TFG_PAIR_HOME_OUTER, once a kernel of its own, is
@@ -306,9 +306,9 @@ TFG_API int tfg_set_pair_lists(tfg_engine *eng, int enable);
 #define TFG_PAIR_HOME_OUTER 32
 TFG_API int tfg_autotune(tfg_engine *eng, int *split);
 TFG_API int tfg_set_split(tfg_engine *eng, int split);
-/* The whole tuple the autotuner picks: the split (as above), the warps per CTA of the tiled
- * kernel (8, or 4 for engines whose potentials are all tabulated: twice the CTAs per SM) and
- * the home cells a warp takes from the shared work counter at a time (1..8; it times 1, 2, 4).
+/* The whole tuple the autotuner picks: the split (as above), the warps per CTA (8 or, for engines
+ * whose potentials are all tabulated, 4: accepted, without effect, the size of the work items
+ * decides) and the fewest work items a warp takes from the shared counter at a time (1..8).
  * The reference's counterparts are the hand-set blocks and threads of
  * cuda::EngineConfig::setBlocks / setThreads (source/cuda/tfEngineConfig.cpp:98-124). */
 TFG_API int tfg_get_tuning(tfg_engine *eng, int *split, int *warps_per_cta, int *grab);

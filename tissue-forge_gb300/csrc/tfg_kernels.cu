@@ -196,8 +196,8 @@ __global__ void k_relocate(int n, int src0, int dst0, int cap_src, int cap_dst, 
     }
 }
 
-// Binning, in four launches (one for small arenas, k_bin_small).  It is bound by launches and L2 latency below about 100,000
-// particles and by HBM above:
+// Binning, in four launches (one for small arenas, k_bin_small).  It is bound by launches and L2
+// latency below about 100,000 particles and by HBM above:
 //   k_bin_count    re-check of the cell-relative positions, count per cell
 //   k_scan         block-local scan of the counts; the last block to finish scans the block
 //                  totals; the simulations' tick
@@ -239,7 +239,7 @@ __global__ void k_bin_count(int n, int nsims, const SimParams *sims, const int32
     stamp_begin(stamp);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int c = i < n ? recheck(i, nsims, sims, cell_sim, pos, cell, shuffle) : -1;
-    // neighbouring particles mostly share a cell: one atomic per warp and cell (25 -> 12 us on
+    // neighbouring particles mostly share a cell: one atomic per warp and cell (25 -> 17 us on
     // 2,000,000 particles at 13 a cell)
     const unsigned same = __match_any_sync(0xffffffffu, c);
     const int lane = threadIdx.x & 31, leader = __ffs(same) - 1;
@@ -278,9 +278,9 @@ __device__ __forceinline__ unsigned long long block_scan2(unsigned long long v, 
 }
 
 // Work items of the tiled pair pass from four consecutive cells with m[] particles: runs of
-// neighbouring cells along z (column[k]: cell k is the first of a column) while they hold at most `homes` particles together, or single cells (runs false); a crowded cell is
-// several items.  emit(cell, cells, first home particle, item) is called for each; returns their
-// number.
+// neighbouring cells along z (column[k]: cell k is the first of a column) while they hold at most
+// `homes` particles together, or single cells (runs false); a crowded cell is several items.
+// emit(cell, cells, first home particle, item) is called for each; returns their number.
 template <class F>
 __device__ __forceinline__ int cell_items(const int *m, uchar4 column, int homes, bool runs, F emit) {
     if (!runs) {
