@@ -84,6 +84,8 @@ struct SimParams {
     // component of it and of the reference's (x_i - shift) - x_k is rounded at a magnitude of
     // at most five cell edges h (a work item spans four cells along z), so the squares at the
     // cutoff differ by less than 3e-6 h/cutoff + 5e-7 relative; the bound keeps four times that.
+    // Both start from the same shift, which across a face is rounded at the magnitude of the box;
+    // along z the filter adds to it the offset of the item's cell that it starts from.
     float cut_hi;
     float dt, dt_flux;
     float maxx[3], maxx2[3], maxv[3], maxv2[3], h2[3];
