@@ -841,7 +841,9 @@ int bin(tfg_engine *eng, int shuffle, bool timed) {
     b.has_rand = eng->has_rand;
     b.rforce = eng->rforce;
     b.force = eng->force;
-    b.oldx = eng->oldx;
+    // (only a step takes reference positions: after the advance, verlet_rebuild still names the
+    // step that is over)
+    b.oldx = shuffle ? eng->oldx : nullptr;
     if (b.ncells == 0) return TFG_OK;
     launch_bin(b, eng->stream);
     eng->cur ^= 1;
@@ -1068,10 +1070,6 @@ int run_steps(tfg_engine *eng, int nsteps) {
     return TFG_OK;
 }
 
-// Pick the tiled pair kernel's work split (warps per home cell) by timing each choice on
-// the current binned state.  Every trial re-initialises the forces with a non-shuffling
-// re-bin (idempotent on sorted data); the flux increments the trials add are saved and
-// restored, so the engine state is unchanged.
 int tune_if_needed(tfg_engine *eng) {
     if (eng->split == 0) return autotune(eng);
     // A batch whose population changed by more than 4x since the autotuner ran (a served
@@ -1080,6 +1078,10 @@ int tune_if_needed(tfg_engine *eng) {
     return TFG_OK;
 }
 
+// Pick the tiled pair kernel's work split (warps per home cell) by timing each choice on
+// the current state.  Every trial re-initialises the forces with a non-shuffling re-bin.  What the
+// trials change is kept and put back, by particle id: after a step the first re-bin moves the
+// particles that have left their cell to other slots.  So the engine state is unchanged.
 int autotune(tfg_engine *eng, bool splits_only) {
     if (!use_tile(eng) || eng->n == 0) {
         eng->split = 1;
@@ -1088,11 +1090,19 @@ int autotune(tfg_engine *eng, bool splits_only) {
         return TFG_OK;
     }
     cudaStream_t s = eng->stream;
-    const size_t nq = (size_t)eng->cap * std::max(1, eng->nspec);
-    float *save = nullptr;
-    int rc = dalloc(eng, &save, nq);
-    if (rc) return rc;
-    CK(cudaMemcpyAsync(save, eng->A[eng->cur].sq, sizeof(float) * nq, cudaMemcpyDeviceToDevice, s));
+    const size_t nred = eng->order.size() * RED_COUNT;
+    struct Kept {
+        float4 *force = nullptr;
+        float *sq = nullptr;
+        double *red = nullptr;
+        ~Kept() { cudaFree(force); cudaFree(sq); cudaFree(red); }
+    } kept;
+    int rc;
+    if ((rc = dalloc(eng, &kept.force, eng->n)) || (rc = dalloc(eng, &kept.sq, (size_t)eng->n * eng->nspec)) ||
+        (rc = dalloc(eng, &kept.red, nred)))
+        return rc;
+    launch_keep(eng->n, eng->cap, eng->nspec, false, eng->A[eng->cur], eng->force, kept.force, kept.sq, s);
+    CK(cudaMemcpyAsync(kept.red, eng->red, sizeof(double) * nred, cudaMemcpyDeviceToDevice, s));
     // candidates: every work split of the tiled kernel (it sizes its grabs itself)
     std::vector<TileTune> cand;
     for (int split : {1, 2, 7, 14}) {
@@ -1122,10 +1132,10 @@ int autotune(tfg_engine *eng, bool splits_only) {
     // twice more and the best of their times decides
     std::vector<float> once(cand.size());
     for (size_t c = 0; c < cand.size(); c++) {
-        if ((once[c] = trial(cand[c])) < 0.f) { cudaFree(save); return rc; }
+        if ((once[c] = trial(cand[c])) < 0.f) return rc;
         for (int rep = 0; rep < 2 && once[c] < 0.5f; rep++) {
             const float ms = trial(cand[c]);
-            if (ms < 0.f) { cudaFree(save); return rc; }
+            if (ms < 0.f) return rc;
             once[c] = std::min(once[c], ms);
         }
     }
@@ -1140,16 +1150,14 @@ int autotune(tfg_engine *eng, bool splits_only) {
         float tmin = once[order[k]];
         for (int rep = 0; rep < 2; rep++) {
             const float ms = trial(cand[order[k]]);
-            if (ms < 0.f) { cudaFree(save); return rc; }
+            if (ms < 0.f) return rc;
             tmin = std::min(tmin, ms);
         }
         if (tmin < best) { best = tmin; best_t = cand[order[k]]; }
     }
-    CK(cudaMemcpyAsync(eng->A[eng->cur].sq, save, sizeof(float) * nq, cudaMemcpyDeviceToDevice, s));
-    CK(cudaStreamSynchronize(s));
-    cudaFree(save);
-    rc = bin(eng, 0);
-    if (rc) return rc;
+    if ((rc = bin(eng, 0))) return rc;
+    launch_keep(eng->n, eng->cap, eng->nspec, true, eng->A[eng->cur], eng->force, kept.force, kept.sq, s);
+    CK(cudaMemcpyAsync(eng->red, kept.red, sizeof(double) * nred, cudaMemcpyDeviceToDevice, s));
     CK(cudaStreamSynchronize(s));
     eng->split = best_t.split;
     eng->tune_warps = best_t.warps;

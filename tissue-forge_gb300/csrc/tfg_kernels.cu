@@ -985,6 +985,22 @@ __global__ void k_gather(int n, int slot0, int cap, int nspec, SimParams P, Part
     }
 }
 
+// Forces, densities and flux increments of every particle, kept by its id over binnings that move
+// it to another slot, and put back.
+__global__ void k_keep(int n, int cap, int nspec, bool restore, const float4 *aux, float4 *force, float *sq,
+                       float4 *kept_force, float *kept_sq) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int id = __float_as_int(aux[i].w);
+    if (restore) force[i] = kept_force[id];
+    else kept_force[id] = force[i];
+    for (int s = 0; s < nspec; s++) {
+        const size_t a = (size_t)s * cap + i, b = (size_t)s * n + id;
+        if (restore) sq[a] = kept_sq[b];
+        else kept_sq[b] = sq[a];
+    }
+}
+
 inline int nblk(long long n, int t) { return (int)((n + t - 1) / t); }
 
 }  // namespace
@@ -1008,6 +1024,12 @@ void launch_relocate(int n, int src0, int dst0, int cap_src, int cap_dst, int ns
     if (n > 0)
         k_relocate<<<nblk(n, kThreads), kThreads, 0, s>>>(n, src0, dst0, cap_src, cap_dst, nspec, did, dcell, src,
                                                           dst);
+}
+
+void launch_keep(int n, int cap, int nspec, bool restore, const ParticleArrays &A, float4 *force, float4 *kept_force,
+                 float *kept_sq, cudaStream_t s) {
+    if (n > 0)
+        k_keep<<<nblk(n, kThreads), kThreads, 0, s>>>(n, cap, nspec, restore, A.aux, force, A.sq, kept_force, kept_sq);
 }
 
 int scan_blocks(int ncells) { return nblk(ncells, kScanCells); }

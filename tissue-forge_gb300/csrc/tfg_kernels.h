@@ -45,6 +45,9 @@ void launch_setpartp(int n, const float *xg, const SimParams &P, float3 lo, floa
                      cudaStream_t s);
 void launch_relocate(int n, int src0, int dst0, int cap_src, int cap_dst, int nspec, int did, int dcell,
                      const ParticleArrays &src, const ParticleArrays &dst, cudaStream_t s);
+// Keep the forces and flux increments of ids [0, n) in kept_force (n) and kept_sq (nspec x n), or put them back.
+void launch_keep(int n, int cap, int nspec, bool restore, const ParticleArrays &A, float4 *force, float4 *kept_force,
+                 float *kept_sq, cudaStream_t s);
 void launch_bin(const BinArgs &b, cudaStream_t s);
 void launch_bonds(int nb, int sms, const SimParams *sims, const int32_t *cell_sim, const int2 *bonds, const int32_t *bslot,
                   const PotDev *bpots, const float *bblob, const int32_t *slot_of_id, const float4 *pos,
