@@ -1,0 +1,25 @@
+// Calls the launch functions of the binning and the pair pass as an engine does.
+#include <cstring>
+
+#include "tfg_kernels.h"
+
+namespace tfg {
+void launch_pair_stencil_fluxonly(const PairKernelArgs &, cudaStream_t) {}
+}  // namespace tfg
+
+// One binning and one pair pass of n particles in `cells` cells.
+extern "C" void drive_step(int n, int cells, int homes, int dpd, int sms) {
+    tfg::BinArgs b;
+    std::memset(static_cast<void *>(&b), 0, sizeof(b));
+    b.n = n;
+    b.ncells = cells;
+    b.homes = homes;
+    tfg::launch_bin(b, nullptr);
+    tfg::PairKernelArgs a;
+    std::memset(&a, 0, sizeof(a));
+    a.n = n;
+    a.ncells = cells;
+    a.homes = homes;
+    a.runs = a.has_dpd = dpd != 0;
+    tfg::launch_pair_tile(a, sms, false, tfg::TileTune(), nullptr);
+}

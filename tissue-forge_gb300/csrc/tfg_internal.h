@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <string>
 #include <vector>
 
@@ -40,6 +41,25 @@ inline void launch_step_kernel(void (*kernel)(P...), int grid, int block, size_t
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
+
+// A kernel's set-up, made once on each device that it is launched on: function attributes and
+// occupancy are a device's.  make() returns a positive number that is kept (resident warps, say),
+// or 0 after an error, which the check of the launch reports; it may run twice when two threads
+// are first at once.
+class PerDevice {
+public:
+    template <class F> int get(F make) {
+        int d = 0;
+        if (cudaGetDevice(&d) != cudaSuccess || d < 0 || d >= kDevices) return make();
+        int n = kept[d].load(std::memory_order_relaxed);
+        if (n == 0) kept[d].store(n = make(), std::memory_order_relaxed);
+        return n;
+    }
+
+private:
+    static constexpr int kDevices = 64;
+    std::atomic<int> kept[kDevices] = {};
+};
 
 // Reduction slots in the device double array.
 enum RedSlot : int {

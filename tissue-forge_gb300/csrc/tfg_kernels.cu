@@ -1036,9 +1036,11 @@ int scan_blocks(int ncells) { return nblk(ncells, kScanCells); }
 
 template <bool kExt, bool kRand> void launch_bin_variant(const BinArgs &b, cudaStream_t s) {
     if (b.n <= kSmallBlocks * kSmallThreads && b.ncells <= kSmallCells) {
-        static const cudaError_t attr = cudaFuncSetAttribute(
-            k_bin_small<kExt, kRand>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallCells * (int)sizeof(int32_t));
-        (void)attr;   // a failure shows at the launch
+        static PerDevice ready;
+        ready.get([] {
+            return cudaFuncSetAttribute(k_bin_small<kExt, kRand>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        kSmallCells * (int)sizeof(int32_t)) == cudaSuccess;
+        });
         launch_step_kernel(k_bin_small<kExt, kRand>, kSmallBlocks, kSmallThreads, sizeof(int32_t) * kSmallCells, s, b);
         return;
     }
