@@ -306,9 +306,9 @@ TFG_API int tfg_set_pair_lists(tfg_engine *eng, int enable);
 #define TFG_PAIR_HOME_OUTER 32
 TFG_API int tfg_autotune(tfg_engine *eng, int *split);
 TFG_API int tfg_set_split(tfg_engine *eng, int split);
-/* The whole tuple the autotuner picks: the split (as above), the warps per CTA (8 or, for engines
- * whose potentials are all tabulated, 4: accepted, without effect, the size of the work items
- * decides) and the fewest work items a warp takes from the shared counter at a time (1..8).
+/* The launch shape of the pair pass: the split (as above), the warps per CTA (4 or 8; by the size
+ * of the work items unless tfg_set_tuning has fixed it) and the fewest work items a warp takes from
+ * the shared counter at a time (1..8).
  * The reference's counterparts are the hand-set blocks and threads of
  * cuda::EngineConfig::setBlocks / setThreads (source/cuda/tfEngineConfig.cpp:98-124). */
 TFG_API int tfg_get_tuning(tfg_engine *eng, int *split, int *warps_per_cta, int *grab);

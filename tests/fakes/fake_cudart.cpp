@@ -9,7 +9,7 @@ namespace {
 int device = 0;
 std::map<std::pair<int, const void *>, int> shared_limit;   // opt-in, per device and kernel
 int launches = 0, refused = 0;
-unsigned last_grid = 0;
+unsigned last_grid = 0, last_block = 0;
 }  // namespace
 
 extern "C" {
@@ -17,6 +17,7 @@ void fake_set_device(int d) { device = d; }
 int fake_launches() { return launches; }
 int fake_refused() { return refused; }
 unsigned fake_last_grid() { return last_grid; }
+unsigned fake_last_block() { return last_block; }
 
 cudaError_t cudaGetDevice(int *d) {
     *d = device;
@@ -34,6 +35,7 @@ cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int *n, const
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *f, void **) {
     launches++;
     last_grid = c->gridDim.x;
+    last_block = c->blockDim.x;
     const auto it = shared_limit.find({device, f});
     if (c->dynamicSmemBytes > 48 * 1024 && (it == shared_limit.end() || (size_t)it->second < c->dynamicSmemBytes)) {
         refused++;

@@ -7,8 +7,8 @@ namespace tfg {
 void launch_pair_stencil_fluxonly(const PairKernelArgs &, cudaStream_t) {}
 }  // namespace tfg
 
-// One binning and one pair pass of n particles in `cells` cells.
-extern "C" void drive_step(int n, int cells, int homes, int dpd, int sms) {
+// One binning and one pair pass of n particles in `cells` cells (warps per CTA 0: by rule).
+extern "C" void drive_step(int n, int cells, int homes, int dpd, int warps, int sms) {
     tfg::BinArgs b;
     std::memset(static_cast<void *>(&b), 0, sizeof(b));
     b.n = n;
@@ -21,5 +21,7 @@ extern "C" void drive_step(int n, int cells, int homes, int dpd, int sms) {
     a.ncells = cells;
     a.homes = homes;
     a.runs = a.has_dpd = dpd != 0;
-    tfg::launch_pair_tile(a, sms, false, tfg::TileTune(), nullptr);
+    tfg::TileTune t;
+    t.warps = warps;
+    tfg::launch_pair_tile(a, sms, false, t, nullptr);
 }

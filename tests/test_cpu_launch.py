@@ -14,7 +14,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 OUT = os.path.join(HERE, "fakes", "_build", "libtfg_launch.so")
 
 
-@pytest.fixture()
+@pytest.fixture(scope="module")
 def fake():
     cuda = os.path.dirname(os.path.dirname(tfg_build.NVCC))
     inc = ["-I" + os.path.join(tfg_build.HERE, "csrc"), "-I" + os.path.join(tfg_build.ROOT, "include")]
@@ -33,7 +33,15 @@ def test_kernels_are_set_up_on_every_device(fake):
         fake.fake_set_device(device)
         for n, cells, homes, dpd in ((500, 125, 8, 0), (50_000, 20_000, 16, 0), (5_000, 8_000, 8, 1), (2_000_000, 150_000, 32, 0)):
             before = fake.fake_launches()
-            fake.drive_step(n, cells, homes, dpd, 152)
+            fake.drive_step(n, cells, homes, dpd, 0, 152)
             assert fake.fake_launches() > before
             assert fake.fake_refused() == 0, (device, n)
         assert fake.fake_last_grid() == 152 * per_sm
+
+
+@pytest.mark.parametrize("dpd", [0, 1])
+def test_warps_of_a_block(fake, dpd):
+    """By the home particles of a work item, or as the caller fixes them."""
+    for homes, warps, threads in ((8, 0, 128), (16, 0, 128), (32, 0, 256), (8, 8, 256), (32, 4, 128), (32, 8, 256)):
+        fake.drive_step(100_000, 20_000, homes, dpd, warps, 152)
+        assert fake.fake_last_block() == threads, (homes, warps)

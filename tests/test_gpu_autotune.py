@@ -1,5 +1,5 @@
 """The autotuner on an engine that has stepped: it leaves the state as it was, also where
-particles have moved to cells that the arena is not sorted by yet."""
+particles have moved to cells that the arena is not sorted by yet.  The reported launch shape."""
 import numpy as np
 import pytest
 
@@ -68,3 +68,21 @@ def test_autotune_keeps_the_verlet_reference_positions():
     assert rg == rh == 1
     # positions of the two runs differ by the rounding of force sums taken in another order
     assert abs(mg - mh) <= 1e-3 * mh
+
+
+@pytest.mark.parametrize("name,n,warps", [("cells", 3000, 4), ("cells", 120_000, 8), ("dpd", 120_000, 4)])
+def test_tuning_reports_the_warps_of_a_block(name, n, warps):
+    """Blocks have four warps where work items are small (up to 16 home particles), else eight, and
+    what the caller fixes."""
+    w = configs.cell_sorting(n=n, side=float((2 * n) ** (1 / 3)), seed=3) if name == "cells" else \
+        configs.dpd_droplets(n=n, side=42.5, radius=12.75, seed=3)
+    g = make_gpu(w)
+    g.autotune()
+    assert g.tuning()[1] == warps
+    g.set_tuning(1, 12 - warps, 1)
+    g.force_only()
+    assert g.tuning() == (1, 12 - warps, 1)
+    f = g.download()["density"]
+    g = make_gpu(w)
+    g.force_only()
+    assert np.abs(f - g.download()["density"]).max() <= 1e-5 * f.max()

@@ -538,7 +538,7 @@ TFG_API int tfg_get_verlet(tfg_engine *eng, int64_t *rebuilds, float *maxdx) {
 TFG_API int tfg_get_tuning(tfg_engine *eng, int *split, int *warps, int *grab) {
     if (!eng) return TFG_E_INVAL;
     if (split) *split = eng->split;
-    if (warps) *warps = eng->tune_warps;
+    if (warps) *warps = cta_warps(tune_of(eng), eng->homes);
     if (grab) *grab = eng->tune_grab;
     return TFG_OK;
 }

@@ -137,7 +137,7 @@ struct tfg_engine {
     int split = 0;                   // tiled pair pass: warps per home cell (0 = not tuned)
     bool tune_auto = false;          // the tuple is the autotuner's (not fixed by the caller)
     int64_t tuned_n = 0;             // particles when the autotuner last ran
-    int tune_warps = 8;              // tiled pair pass: warps per CTA (table variants: 8 or 4)
+    int tune_warps = 0;              // tiled pair pass: warps per CTA (8 or 4; 0: by the work items)
     int tune_grab = 1;               // tiled pair pass: work items per grab
     bool deterministic = false;      // pair pass without atomics (stencil kernel): reproducible bits
     int capacity_hint = 0;

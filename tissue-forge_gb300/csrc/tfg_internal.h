@@ -132,15 +132,19 @@ struct PairKernelArgs {
 // Full-stencil kernel: one thread per particle, no atomics.  General path (any number
 // of species); force[] must hold the initial force (external + random, density W(0)).
 void launch_pair(const PairKernelArgs &a, cudaStream_t s);
-// Launch configuration of the nonbonded pass, picked by the autotuner: the work split (warps
+// Launch configuration of the nonbonded pass: the work split picked by the autotuner (warps
 // per home cell: 1, 2, 7 or 14; the cell's 14 tasks are divided into that many work items;
-// TFG_PAIR_HOME_OUTER means 1), the warps per CTA (kept for callers; every CTA has 8), and the
-// fewest work items a warp takes from the shared counter at a time.
+// TFG_PAIR_HOME_OUTER means 1), the warps per CTA (4 or 8; 0: by the size of the work items),
+// and the fewest work items a warp takes from the shared counter at a time.
 struct TileTune {
     int split = 1;
-    int warps = 8;
+    int warps = 0;
     int grab = 1;
 };
+// Warps per CTA of the tiled pass.  CTAs of four end more evenly where a warp has few items: 76.7 ->
+// 74.6 us a step of 100,000 DPD particles, 70.4 -> 69.3 of 80,000 cells; CTAs of eight share more
+// in L1: 703 us a step of 1,953,125 Lennard-Jones particles, 709 with four.
+inline int cta_warps(const TileTune &t, int homes) { return t.warps ? t.warps : (homes < 32 ? 4 : 8); }
 // Tiled half-shell kernel; force[] must hold the initial force, to which both partners'
 // contributions are added atomically.
 void launch_pair_tile(const PairKernelArgs &a, int sms, bool signature, const TileTune &tune, cudaStream_t s);
