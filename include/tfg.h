@@ -296,7 +296,7 @@ TFG_API int tfg_set_graphs(tfg_engine *eng, int enable);
 TFG_API int tfg_set_pair_lists(tfg_engine *eng, int enable);
 /* Autotune the nonbonded pass's form by timing each choice on the current state; the
  * state is left unchanged.  The choices are the tiled kernel's work split (warps per home
- * cell: 1, 2, 7 or 14).  tfg_step and
+ * cell: 1, 2, 7 or 14); large arenas in Verlet mode take 1 without trials.  tfg_step and
  * tfg_force_only run it on their first call, and time the work splits again whenever the
  * particle count has grown or shrunk more than 4x since (a batch that fills up or drains);
  * tfg_set_split fixes the choice instead (TFG_PAIR_HOME_OUTER, once a kernel of its own, is

@@ -1083,7 +1083,14 @@ int tune_if_needed(tfg_engine *eng) {
 // trials change is kept and put back, by particle id: after a step the first re-bin moves the
 // particles that have left their cell to other slots.  So the engine state is unchanged.
 int autotune(tfg_engine *eng, bool splits_only) {
-    if (!use_tile(eng) || eng->n == 0) {
+    // Arenas on tables whose simulations are all in Verlet mode take split 1 from 12,000 particles
+    // on.  Trials double the time from the load to the first step there (2.5 ms without, 5.6 with
+    // them on 262,144 particles, 6.4 and 12.7 on 1,000,000) and find nothing better: a step with
+    // splits 1 and 2 takes 28.5 and 27.6 us on 8,000 particles, 39.5 and 41.3 on 15,625, 44.2 and
+    // 47.4 on 32,768, 62.1 and 64.8 on 64,000 (skin 0.2 cutoffs; with 0.5, 79.6 and 76.7 on 64,000).
+    bool verlet = !eng->has_dpd && !(eng->has_flux && eng->nspec > 0) && eng->n >= 12000;
+    for (int k : eng->order) verlet &= (eng->sims[k].P.flags & TFG_ENGINE_VERLET) != 0;
+    if (!use_tile(eng) || eng->n == 0 || verlet) {
         eng->split = 1;
         eng->tune_auto = true;
         eng->tuned_n = eng->n;
