@@ -793,16 +793,24 @@ int load_sim(tfg_engine *eng, int sim, int n, const float *xg, const int32_t *ce
 
 // Work items of the tiled pass: the most home particles of one, and whether one may span several
 // cells.  A small arena leaves warps without an item, and its time is that of the longest one,
-// a crowded cell's: with 8, 16 and 32 home particles the pass takes 12, 14 and 20 us on 2,000
-// clustered cells, 20, 22 and 32 on 20,000.  Larger items share more: the step takes 89, 81 and
-// 86 us on 100,000 uniform cells, 106, 96 and 97 on 150,000, 117 and 115 (16, 32) on 200,000,
-// 150 and 141 on 300,000; 73 and 72 on an LJ fluid of 110,592.  DPD pairs cost more each and
-// droplets spread out, so that balance counts at every size: 82, 77 and 81 us on 100,000
-// particles, 161 and 173 on 300,000, 967 and 1007 on 2,000,000.
-// Runs of cells share set-up and targets, most where cells hold few particles (DPD droplets
-// that have spread out: 77 -> 38 us), but leave fewer items: without and with them 141 and 144 us
-// on 300,000 uniform cells, 185 and 179 on 400,000; 147 and 151 on LJ fluids of 343,000
-// particles, 178 and 174 on 421,875.
+// a crowded cell's; larger items share more.  Particles stand for the items a warp gets: of that,
+// kinds of systems differ, so that each line lies among the sizes where the two sides meet.
+// Microseconds a step, each side with the work split that is best for it:
+//   8 or 16 homes, 24,000       cells 20,000 40.3 43.8, 24,000 46.6 46.2, 32,000 50.6 47.9; LJ fluids
+//                               20,000 38.0 35.7, 33,000 48.3 43.8; DPD 10,000 35.7 35.8, 24,000
+//                               44.1 39.7, 28,000 44.7 46.4, 50,000 53.8 54.1, 80,000 69.4 63.3
+//   16 or 32, tables, 110,000   LJ 80,000 61.2 62.4, 110,592 72.4 72.2, 148,877 84.2 81.1; cells 80,000
+//                               67.0 75.2, 110,000 78.0 82.1, 130,000 86.6 86.7, 150,000 94.5 93.2,
+//                               200,000 109.7 107.2, 300,000 142.0 132.0
+//   16 or 32, DPD, never        100,000 particles 77 81, 200,000 109.3 107.7, 300,000 146.5 149.8,
+//                               400,000 198.5 193.6, 2,000,000 967 1007: pairs cost more each and
+//                               droplets spread out, so that balance counts at every size
+//   32 without or with runs     cells 300,000 132.0 136.6, 400,000 164.0 167.2, 450,000 186.8 181.7,
+//   of cells, tables, 400,000   600,000 232.3 232.1, 2,000,000 696.6 681.4; LJ 300,763 129.6 127.8,
+//                               405,224 165.1 160.5, 1,000,000 365.1 349.5; 80 and 256 tissues of 0.7
+//                               and 3.0 million cells 281.9 282.7, 1,115.6 1,092.1
+// Runs share set-up and targets, most where cells hold few particles (DPD droplets that have spread
+// out: 77 -> 38 us a pass), but leave fewer items.
 static void plan_items(tfg_engine *eng) {
     const bool pairs_cost = eng->has_dpd || (eng->has_flux && eng->nspec > 0);
     eng->homes = eng->n < 24000 ? 8 : (pairs_cost || eng->n < 110000 ? 16 : 32);
@@ -1074,7 +1082,7 @@ int tune_if_needed(tfg_engine *eng) {
     if (eng->split == 0) return autotune(eng);
     // A batch whose population changed by more than 4x since the autotuner ran (a served
     // batch that filled up or drained) re-times the work split, the knob that follows size.
-    if (eng->tune_auto && (eng->n > 4 * eng->tuned_n || 4 * eng->n < eng->tuned_n)) return autotune(eng, true);
+    if (eng->tune_auto && (eng->n > 4 * eng->tuned_n || 4 * eng->n < eng->tuned_n)) return autotune(eng);
     return TFG_OK;
 }
 
@@ -1082,7 +1090,7 @@ int tune_if_needed(tfg_engine *eng) {
 // the current state.  Every trial re-initialises the forces with a non-shuffling re-bin.  What the
 // trials change is kept and put back, by particle id: after a step the first re-bin moves the
 // particles that have left their cell to other slots.  So the engine state is unchanged.
-int autotune(tfg_engine *eng, bool splits_only) {
+int autotune(tfg_engine *eng) {
     // Arenas on tables whose simulations are all in Verlet mode take split 1 from 12,000 particles
     // on.  Trials double the time from the load to the first step there (2.5 ms without, 5.6 with
     // them on 262,144 particles, 6.4 and 12.7 on 1,000,000) and find nothing better: a step with

@@ -177,13 +177,13 @@ int commit(tfg_engine *eng);                    // re-lay the arena out and uplo
 int bin(tfg_engine *eng, int shuffle, bool timed = false);
 int force_pass(tfg_engine *eng, bool bonded, bool timed);
 int one_step(tfg_engine *eng, bool advance, bool timed);
-void advance_clocks(tfg_engine *eng);           // host clocks, by k_tick's rule (stops included)
+void advance_clocks(tfg_engine *eng);           // host clocks, by tick()'s rule (stops included)
 int set_stop_sim(tfg_engine *eng, int sim, int64_t step);
-int enqueue_step(tfg_engine *eng, bool advance, bool timed);
-int flux_substeps(tfg_engine *eng);  // one_step without the host clock
+int enqueue_step(tfg_engine *eng, bool advance, bool timed);   // one_step without the host clock
+int flux_substeps(tfg_engine *eng);
 int graph_steps(tfg_engine *eng, int steps);    // steps replayed from a captured graph
 int run_steps(tfg_engine *eng, int nsteps);     // nsteps steps, graphs where they apply
-int autotune(tfg_engine *eng, bool splits_only = false);
+int autotune(tfg_engine *eng);
 int tune_if_needed(tfg_engine *eng);   // first tuning, or a re-tune after the batch grew or shrank 4x
 inline TileTune tune_of(const tfg_engine *eng) {
     TileTune t;
